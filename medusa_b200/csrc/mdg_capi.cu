@@ -538,6 +538,14 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
   // layout: state offsets, table offsets, tiles
   std::vector<Tile> tiles, ytiles;
   int64_t cell = 0, rc0 = 0, rc1 = 0, sh = 0;
+  int xrows = TIX2, yrows = TIY2;
+  if (cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) s->num_sms = 0;
+  if (ndim == 2) {
+    std::vector<int> r1, r2;
+    for (int m = 0; m < nprob; m++) { r1.push_back(descs[m].n1); r2.push_back(descs[m].n2); }
+    xrows = tile_rows_2d(0, r1.data(), r2.data(), nprob, s->num_sms);
+    yrows = tile_rows_2d(1, r1.data(), r2.data(), nprob, s->num_sms);
+  }
   for (int m = 0; m < nprob; m++) {
     const mdg_problem_desc &d = descs[m];
     ProbDev P;
@@ -556,10 +564,10 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
     if (d.ndim == 2) {
       rc1 += P.n2 + 2 * NG;
       sh += (int64_t)(P.n1 + 3) * P.n2;
-      for (int i0 = 0; i0 < P.n1; i0 += TIX2)
-        for (int j0 = 0; j0 < P.n2; j0 += NTX2) tiles.push_back(Tile{m, i0, j0, 0});
-      for (int i0 = 0; i0 < P.n1; i0 += TIY2)
-        for (int j0 = 0; j0 < P.n2; j0 += TJY2) ytiles.push_back(Tile{m, i0, j0, 0});
+      for (int i0 = 0; i0 < P.n1; i0 += xrows)
+        for (int j0 = 0; j0 < P.n2; j0 += NTX2) tiles.push_back(Tile{m, i0, j0, xrows});
+      for (int i0 = 0; i0 < P.n1; i0 += yrows)
+        for (int j0 = 0; j0 < P.n2; j0 += TJY2) ytiles.push_back(Tile{m, i0, j0, yrows});
     } else {
       for (int i0 = 0; i0 < P.n1; i0 += TILE1) tiles.push_back(Tile{m, i0, 0, 0});
     }

@@ -29,8 +29,8 @@ struct Tables {
 // number of (problem, tile) items in the tile list.
 struct WorkQueue { unsigned int head[2]; int ntiles; int pad; };
 
-// One work tile: problem, first output row i0, first output column j0 (2-D).
-struct Tile { int prob; int i0; int j0; int pad; };
+// One work tile: problem, first output row i0, first output column j0 and output rows (2-D).
+struct Tile { int prob; int i0; int j0; int rows; };
 
 constexpr int NT1 = 128;          // threads per 1-D tile (126 output zones)
 constexpr int TILE1 = NT1 - 2;
@@ -48,10 +48,13 @@ constexpr int TILE1 = NT1 - 2;
 #define MDG_YMINB 4
 #endif
 constexpr int NTX2 = 128;         // threads (= columns) per direction-0 tile
-constexpr int TIX2 = MDG_TIX2;    // rows per direction-0 tile
+constexpr int TIX2 = MDG_TIX2;    // most rows of a direction-0 tile
 constexpr int NTY2 = 128;         // threads per direction-1 tile (126 output columns)
 constexpr int TJY2 = NTY2 - 2;
-constexpr int TIY2 = MDG_TIY2;    // rows per direction-1 tile
+constexpr int TIY2 = MDG_TIY2;    // most rows of a direction-1 tile
+// Rows per direction-0 (dir = 0) or direction-1 tile for 2-D grids of n1[m] rows x n2[m]
+// columns that are swept by the same launches (mdg_sweep2d.cu).
+int tile_rows_2d(int dir, const int *n1, const int *n2, int n, int num_sms);
 
 struct TmaTables1d;
 // Tabulated EOS on the device (mdg_eos_table.cu): the records f[jy][jr][jt] = {e, log p,

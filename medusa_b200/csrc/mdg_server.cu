@@ -557,6 +557,14 @@ int round_once(mdg_server *s, int *active_out)
     std::vector<Tile> tl, tl_tab, xt, yt;
     s->mono1d = false;
     const bool mixed1d = s->cfg.precision == MDG_PREC_MIXED;
+    // rows per 2-D tile: one choice for all resident 2-D problems (one launch sweeps them)
+    std::vector<int> r1, r2;
+    for (int k = 0; k < s->max_probs; k++) {
+      const Request *r = s->slots[k];
+      if (r && r->desc.ndim == 2 && !is_dendritic(r->desc)) { r1.push_back(r->desc.n1); r2.push_back(r->desc.n2); }
+    }
+    const int xrows = tile_rows_2d(0, r1.data(), r2.data(), (int)r1.size(), s->num_sms);
+    const int yrows = tile_rows_2d(1, r1.data(), r2.data(), (int)r1.size(), s->num_sms);
     for (int k = 0; k < s->max_probs; k++) {
       const Request *r = s->slots[k];
       if (!r || is_dendritic(r->desc)) continue;   // dendritic problems run on their own grids
@@ -567,12 +575,12 @@ int round_once(mdg_server *s, int *active_out)
         continue;
       }
       if (r->desc.ndim == 2) {
-        // the solver's 2-D tiling: direction-0 tiles of TIX2 rows x NTX2 columns,
-        // direction-1 tiles of TIY2 rows x TJY2 columns
-        for (int i0 = 0; i0 < r->desc.n1; i0 += TIX2)
-          for (int j0 = 0; j0 < r->desc.n2; j0 += NTX2) xt.push_back(Tile{k, i0, j0, 0});
-        for (int i0 = 0; i0 < r->desc.n1; i0 += TIY2)
-          for (int j0 = 0; j0 < r->desc.n2; j0 += TJY2) yt.push_back(Tile{k, i0, j0, 0});
+        // the solver's 2-D tiling: direction-0 tiles of xrows rows x NTX2 columns,
+        // direction-1 tiles of yrows rows x TJY2 columns
+        for (int i0 = 0; i0 < r->desc.n1; i0 += xrows)
+          for (int j0 = 0; j0 < r->desc.n2; j0 += NTX2) xt.push_back(Tile{k, i0, j0, xrows});
+        for (int i0 = 0; i0 < r->desc.n1; i0 += yrows)
+          for (int j0 = 0; j0 < r->desc.n2; j0 += TJY2) yt.push_back(Tile{k, i0, j0, yrows});
       } else {
         for (int i0 = 0; i0 < r->desc.n1; i0 += s->tile_len) tl.push_back(Tile{k, i0, 0, 0});
       }

@@ -152,7 +152,7 @@ xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
   constexpr int RING = MIX ? 5 : 4;
   // column stencil ring (rows r-1 .. r+2 of this thread's column), fed by cp.async
   __shared__ double ring[RING][6][NTX2];
-  // direction-0 reconstruction coefficients of rows i0-1 .. i0+TIX2
+  // direction-0 reconstruction coefficients of rows i0-1 .. i0+rows (at most TIX2 rows)
   __shared__ double xrc[RC_NFIELDS][TIX2 + 2];
   __shared__ float xmx[MIX ? MX_NFIELDS : 1][TIX2 + 2];
   __shared__ double sred[32];
@@ -163,7 +163,7 @@ xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
   const int t = threadIdx.x;
   const int j = tile.j0 + t;
   const int i0 = tile.i0;
-  const int ilast = min(i0 + TIX2, n1);           // last face row of this tile (<= n1)
+  const int ilast = min(i0 + tile.rows, n1);      // last face row of this tile (<= n1)
   const bool col_ok = j < n2;
   const int order = P.interp_order;
   const GamConst<double> gc = gam_const(P.gam);
@@ -173,15 +173,16 @@ xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
   // ring slot of a row (rows >= i0-2)
   auto slot = [&](int row) { return MIX ? (row - i0 + 2) % RING : (row & 3); };
 
-  for (int k = t; k < RC_NFIELDS * (TIX2 + 2); k += NTX2) {
-    const int f = k / (TIX2 + 2), rr = k - f * (TIX2 + 2);
-    const int row = min(i0 - 1 + rr, n1);
+  const int nrow = ilast - i0 + 2;                 // table rows i0-1 .. ilast
+  for (int k = t; k < RC_NFIELDS * nrow; k += NTX2) {
+    const int f = k / nrow, rr = k - f * nrow;
+    const int row = i0 - 1 + rr;
     xrc[f][rr] = __ldg(tb.rc0 + f * tb.rc0_stride + P.geo_off + row + NG);
   }
   if (MIX) {
-    for (int k = t; k < MX_NFIELDS * (TIX2 + 2); k += NTX2) {
-      const int f = k / (TIX2 + 2), rr = k - f * (TIX2 + 2);
-      const int row = min(i0 - 1 + rr, n1);
+    for (int k = t; k < MX_NFIELDS * nrow; k += NTX2) {
+      const int f = k / nrow, rr = k - f * nrow;
+      const int row = i0 - 1 + rr;
       xmx[f][rr] = __ldg(tb.mx + f * tb.rc0_stride + P.geo_off + row + NG);
     }
   }
@@ -323,7 +324,7 @@ ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
   const unsigned char *s1 = shock1 + P.sh_off;
   const bool real_col = (jx >= 0) && (jx < n2);
   const bool out_col = (t >= 1) && (t <= NTY2 - 2) && (jx < n2);
-  const int iend = min(tile.i0 + TIY2, n1);
+  const int iend = min(tile.i0 + tile.rows, n1);
   double smax = 0.0;      // max |signal speed| of this thread's faces
   double nmin = 1.0e300;  // min numerator of the source-term limits (zero sources)
   double lsrc = 1.0e300;  // min source-term limit (fixed gravity)
@@ -477,6 +478,37 @@ ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
   lmin = tmin(lmin, lsrc);
   if (STAGE == 1) lmin = tmin(lmin, 1.0 / lmax);
   block_min_to(lmin, &times[tile.prob].minacc, sred);
+}
+
+// Rows per tile.  A tile marches down its rows one after the other, so its time is that of
+// its rows (and of what it does once: two more reconstructed rows in direction 0, the
+// column tables in direction 1), and a row takes a nearly fixed time while few CTAs share
+// an SM (a chain of dependent FP64 operations) and a time that grows with them once four
+// do.  Measured on a B200, plain FP64: a direction-0 row 6.5 us alone on its SM and 11 us
+// beside three others, a direction-1 row 13 us and 14 us.  The count with the smallest
+// modelled time is taken: full-size grids keep the longest tiles (2048^2: 32 and 16 rows),
+// small ones are cut until the chip is full -- 512^2 with 32 and 16 rows gave 64 and 160
+// CTAs for 592 places, and a step took 1.0 ms.
+int tile_rows_2d(int dir, const int *n1, const int *n2, int n, int num_sms)
+{
+  const int most = dir ? TIY2 : TIX2, cols = dir ? TJY2 : NTX2;
+  const double alone = dir ? 13.0 : 6.5, shared = dir ? 3.5 : 2.75, once = dir ? 0.4 : 2.0;
+  const int per_sm = dir ? MDG_YMINB : MDG_XMINB;
+  const int sms = num_sms > 0 ? num_sms : 148;
+  int best = most;
+  double tbest = 0.0;
+  for (int rows = most; rows >= 1; rows--) {
+    long long tiles = 0;
+    for (int m = 0; m < n; m++) tiles += (long long)((n1[m] + rows - 1) / rows) * ((n2[m] + cols - 1) / cols);
+    const long long wave = (long long)per_sm * sms, full = tiles / wave, rest = tiles - full * wave;
+    auto row_time = [&](long long k) { return k <= 0 ? 0.0 : (k * shared > alone ? k * shared : alone); };
+    const double t = (rows + once) * ((double)full * row_time(per_sm) + row_time((rest + sms - 1) / sms));
+    if (rows == most || t < 0.97 * tbest) {
+      best = rows;
+      tbest = t;
+    }
+  }
+  return best;
 }
 
 void launch_stage2d(int stage, bool mixed, const ProbDev *probs, ProbTime *times, const Tile *xtiles, int nxt,
