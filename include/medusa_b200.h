@@ -236,9 +236,10 @@ int mdg_write_timers(mdg_solver *s, int prob, const char *path);
  *                    per SM that pull (problem, tile) items from a device work queue;
  *   steps_per_graph  steps captured in one CUDA graph and replayed by mdg_step
  *                    (0 = direct launches; timing enabled always launches directly);
- *   run_length       dendritic (3-D and 2-D spherical) sweeps: radial and theta faces
- *                    one thread walks per work item, 1..64 (default 16); the results do
- *                    not depend on it;
+ *   run_length       dendritic (3-D and 2-D spherical) sweeps: most radial and theta faces
+ *                    one thread walks per work item, 1..64 (default 16; a grid too small to
+ *                    fill the device with runs this long is cut into shorter ones); the
+ *                    results do not depend on it;
  *   lanes            mixed 1-D sweep: the problems split into 1..4 groups of about equal
  *                    zone count, each group's steps queued on a stream of its own, so that
  *                    one group's short kernels and kernel tails overlap another's stage

@@ -42,11 +42,11 @@ struct PushRow3 {
   int64_t f0i;      // first direction-0 face of row (i, j)
   int64_t f1o, f1i; // first direction-1 face of rows (i, j+1) and (i, j)
   int64_t f2;       // first direction-2 face of row (i, j) (3-D grids)
-  int64_t cell;     // first zone of row (i, j)
-  int nf0o;         // outer rows: 1 or 2
-  int nkp[2];       // outer faces per zone of each outer row
-  int mo;           // outer theta faces: 0 one per zone, 1 half of a coarser row's face, 2 two faces
-  int mi;           // inner theta faces: 0 one per zone, 1 halves of two faces
+  int i, j, ij;     // the row and its index in the row tables
+  unsigned char nf0o;     // outer rows: 1 or 2
+  unsigned char nkp[2];   // outer faces per zone of each outer row
+  unsigned char mo; // outer theta faces: 0 one per zone, 1 half of a coarser row's face, 2 two faces
+  unsigned char mi; // inner theta faces: 0 one per zone, 1 halves of two faces
 };
 
 struct Grid3 {
@@ -79,7 +79,10 @@ struct Grid3 {
   double *gmono;              // [n1] monopole gravity at the radial zone centroids (shell masses first)
   double x0;                  // startx[0]
   int mono;                   // GRAV=SPHERICAL_MONOPOLE_GRAV
-  const PushRow3 *prow;       // [nij] push() flux addresses of interior rows
+  const PushRow3 *prow;       // [nrow] push() flux addresses of the interior rows, in zone order
+  const int64_t *rowcell;     // [nrow] first zone of each interior row
+  const int *row0;            // interior row of zone 128 b, for every CTA b of the zone kernels
+  int nrow;                   // interior rows
 };
 
 MDG_HD inline int ilog2(int s)

@@ -38,6 +38,7 @@
 #include "mdg_kernels.cuh"
 #include "mdg_grid3d.cuh"
 #include "mdg_mixed.cuh"
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 #include <string>
@@ -492,17 +493,69 @@ __device__ __forceinline__ bool flag_shock(const Grid3 &g, int i, int jj, int kc
 // face value for face i, its right face value kept for face i+1), where the reference's
 // interp() builds a 4-zone pencil and reconstructs two zones per face.  The values are
 // the same; only their reuse differs.
-// A run of faces along one direction: faces r0 .. r0+nr-1 of the fixed row `row` (the
-// theta row j for direction 0, the radial row i for direction 1), columns k0 .. k0+cnt-1.
-struct Tile3R { int r0, nr, row, k0, cnt; };
-constexpr int RUN0 = 16;          // default faces per work item (mdg_launch_config::run_length)
+//
+// Work list: a run is nr faces r0 .. r0+nr-1 of the fixed row `row` (the theta row j for
+// direction 0, the radial row i for direction 1) in every phi column of the face row.  The
+// columns of all runs, one per thread, stand one after the other in one line of lanes
+// (runs of equal length together): column k of a run is lane l0 + k, CTA b takes lanes
+// 128 b .. 128 b + 127, and first[b] is the run of its first lane.  Rows have 4 phi zones at
+// the poles and 1 on the 2-D grid, so a CTA per row left most threads without work: 1.4
+// active threads per warp instruction on a 2-D 400 x 256 grid (0.75 + 0.83 ms for the two
+// kernels of a stage there).
+struct Run3 { int r0, nr, row, l0; };
+constexpr int RUN0 = 16;          // default of mdg_launch_config::run_length
+
+// Direction-2 faces: up to T2 faces k0 .. k0+cnt-1 of row (i, j) on lanes l0 .. l0+cnt+1 of
+// a CTA, the n-th segment of that CTA (n < SEG2_MAX).
+struct Seg2 { int i, j, k0, cnt, l0, n; };
+constexpr int SEG2_MAX = 18;      // most segments of a CTA (whole rows have at least 5 faces, 7 lanes)
+
+// Which of a CTA's consecutive items (rows, runs, segments; at least one lane each) this
+// thread's lane belongs to: start(q) is the first lane, relative to the CTA's, of its q-th
+// item after the one its first lane belongs to (NT3 where there is none).
+template <typename F>
+__device__ __forceinline__ int item_of_lane(int *sbeg, F start)
+{
+  const int t = (int)threadIdx.x;
+  sbeg[t] = start(1 + t);
+  __syncthreads();
+  int lo = 0;   // items after the first that start at or before this lane (at most NT3-1)
+#pragma unroll
+  for (int s = NT3 / 2; s > 0; s >>= 1)
+    if (sbeg[lo + s - 1] <= t) lo += s;
+  return lo;
+}
+
+// Thread of a zone kernel: the interior row (index into prow and rowcell) of zone c; CTA b
+// takes the zones 128 b .. 128 b + 127 in zone order.
+__device__ __forceinline__ int zone_row(const Grid3 &g, int *sbeg)
+{
+  const int64_t c0 = (int64_t)blockIdx.x * NT3;
+  const int r0 = __ldg(g.row0 + blockIdx.x);
+  return r0 + item_of_lane(sbeg, [&](int q) {
+    const int64_t d = (r0 + q < g.nrow) ? __ldg(g.rowcell + r0 + q) - c0 : (int64_t)NT3;
+    return d < NT3 ? (int)d : NT3;
+  });
+}
+
+// Thread of a run kernel: its run.
+__device__ __forceinline__ Run3 lane_run(const Run3 *__restrict__ runs, int nrun, const int *__restrict__ first, int *sbeg)
+{
+  const int r0 = __ldg(first + blockIdx.x), b0 = (int)blockIdx.x * NT3;
+  const int q = item_of_lane(sbeg, [&](int k) {
+    const int d = (r0 + k < nrun) ? runs[r0 + k].l0 - b0 : NT3;
+    return d < NT3 ? d : NT3;
+  });
+  return runs[r0 + q];
+}
 
 // The RK stage is a run-time argument here (not a template argument as in the other
 // face kernels): both stages then run the same code, which measured faster for stage 1
 // than its own specialisation.
 template <bool MIX>
 __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
-                                                     Grid3 g, const Tile3R *__restrict__ tiles, StateSoA s,
+                                                     Grid3 g, const Run3 *__restrict__ runs, int nrun,
+                                                     const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, unsigned char *__restrict__ own,
                                                      unsigned char *__restrict__ all0, int stage)
 {
@@ -512,13 +565,14 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *_
   __shared__ double win[NS][7][NT3];
   __shared__ double arb[7][NT3];
   __shared__ double sred[32];
+  __shared__ int sbeg[NT3];
   if (times[0].done) return;
   const ProbDev &P = probs[0];
-  const Tile3R t = tiles[blockIdx.x];
-  const int tid = (int)threadIdx.x;
-  const int i0 = t.r0, j = t.row, k = t.k0 + tid;
+  const int tid = (int)threadIdx.x, lane = (int)blockIdx.x * NT3 + tid;
+  const Run3 t = lane_run(runs, nrun, first, sbeg);
   double lmin = 1.0e300;
-  if (tid < t.cnt) {
+  if (lane < nlane) {
+    const int i0 = t.r0, j = t.row, k = lane - t.l0;
     const int64_t rcs = g.n1 + 2 * NG;
     auto slot = [&](int ii) { return (ii - i0 + 2) % NS; };
 #pragma unroll 1
@@ -630,11 +684,12 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *_
 // of radial row i and sub-face column kk whose face rows share their phi resolution
 // mn = min(dks(i, j), dks(i, j-1)) (every pencil entry, theta row jj at that resolution,
 // is then the same for all faces of the run); a thread walks northwards through its
-// column, one new entry and one zone reconstruction per face.  Tile3R fields here:
+// column, one new entry and one zone reconstruction per face.  Run3 fields here:
 // r0 = j0, nr = faces, row = i.
 template <bool MIX>
 __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
-                                                     Grid3 g, const Tile3R *__restrict__ tiles, StateSoA s,
+                                                     Grid3 g, const Run3 *__restrict__ runs, int nrun,
+                                                     const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
                                                      const unsigned char *__restrict__ all0, int stage)
 {
@@ -642,13 +697,14 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *_
   __shared__ double win[NS][7][NT3];
   __shared__ double arb[7][NT3];
   __shared__ double sred[32];
+  __shared__ int sbeg[NT3];
   if (times[0].done) return;
   const ProbDev &P = probs[0];
-  const Tile3R t = tiles[blockIdx.x];
-  const int tid = (int)threadIdx.x;
-  const int j0 = t.r0, i = t.row, kk = t.k0 + tid;
+  const int tid = (int)threadIdx.x, lane = (int)blockIdx.x * NT3 + tid;
+  const Run3 t = lane_run(runs, nrun, first, sbeg);
   double lmin = 1.0e300;
-  if (tid < t.cnt) {
+  if (lane < nlane) {
+    const int j0 = t.r0, i = t.row, kk = lane - t.l0;
     const int64_t cs = g.cols1;
     const int64_t base = g.rc1_base[ilog2(djs(g, i))] + NG;
     auto slot = [&](int jj) { return (jj - j0 + 2) % NS; };
@@ -755,35 +811,52 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *_
 }
 
 // Direction-2 faces: face k in [0, nk] of row (i, j) (step.c:1267-1425), with the
-// polar-axis fix on the last theta row.  A CTA takes NT3-2 consecutive faces of one row:
-// it stages the zones they read in shared memory (each zone loaded once) and
-// reconstructs every zone once (the reference reconstructs each zone for both of its
-// faces), then each thread solves one face.
+// polar-axis fix on the last theta row.  A CTA takes segments of consecutive faces of one
+// row each (Seg2; short rows share a CTA, a long one is cut): per segment it stages the
+// zones they read in shared memory (each zone loaded once) and reconstructs every zone
+// once (the reference reconstructs each zone for both of its faces), then a thread solves
+// one face.  With one row per CTA the 128 x 64 x 128 grid ran 13274 CTAs at 20 active
+// threads per warp instruction (0.36 ms a stage, plain FP64).
 constexpr int T2 = NT3 - 2;
 template <int STAGE, bool MIX>
 __global__ void __launch_bounds__(NT3, MDG_F3MINB) face2_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
-                                                     Grid3 g, const Tile3 *__restrict__ tiles, StateSoA s,
+                                                     Grid3 g, const Seg2 *__restrict__ segs, int nseg,
+                                                     const int *__restrict__ first, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
                                                      const unsigned char *__restrict__ all0)
 {
-  __shared__ double sv[7][T2 + 4];    // zones k0-2 .. k0+cnt+1
-  __shared__ double sal[7][T2 + 2];   // left / right face values of zones k0-1 .. k0+cnt
-  __shared__ double sar[7][T2 + 2];
+  __shared__ double sv_[7][NT3 + 2 * SEG2_MAX];   // zones k0-2 .. k0+cnt+1 of each segment
+  __shared__ double sal_[7][NT3];                 // left / right face values of zones k0-1 .. k0+cnt
+  __shared__ double sar_[7][NT3];
   __shared__ double sred[32];
+  __shared__ int sbeg[NT3];
   if (times[0].done) return;
   const ProbDev &P = probs[0];
-  const Tile3 tl = tiles[blockIdx.x];
+  const int s0 = __ldg(first + blockIdx.x);
+  const Seg2 tl = segs[s0 + item_of_lane(sbeg, [&](int q) {
+    return (q < SEG2_MAX && s0 + q < nseg && segs[s0 + q].n == q) ? segs[s0 + q].l0 : NT3;
+  })];
   const int i = tl.i, j = tl.j, k0 = tl.k0, cnt = tl.cnt;
-  const int t = (int)threadIdx.x;
+  const int t = (int)threadIdx.x - tl.l0;   // lane within the segment; past cnt+1: no work
+  // this segment's part of the shared arrays, indexed by t
+  double (*sv)[NT3 + 2 * SEG2_MAX] = reinterpret_cast<double(*)[NT3 + 2 * SEG2_MAX]>(&sv_[0][tl.l0 + 2 * tl.n]);
+  double (*sal)[NT3] = reinterpret_cast<double(*)[NT3]>(&sal_[0][tl.l0]);
+  double (*sar)[NT3] = reinterpret_cast<double(*)[NT3]>(&sar_[0][tl.l0]);
   const int ij = rowi(g, i, j);
   const int dk = dks(g, i, j);
   const int64_t base = g.rc2_base[ilog2(dk)] + NG;
   const bool pole = (j == nj_of(g, i) - 1);
-  for (int q = t; q < cnt + 4; q += NT3) {
+  if (t < cnt + 2) {
     double w[7];
-    load7(g, P, s, i, j, k0 - 2 + q, w);
+    load7(g, P, s, i, j, k0 - 1 + t, w);
 #pragma unroll
-    for (int v = 0; v < 7; v++) sv[v][q] = w[v];
+    for (int v = 0; v < 7; v++) sv[v][t + 1] = w[v];
+    if (t == 0 || t == cnt + 1) {
+      const int e = t == 0 ? 0 : cnt + 3;
+      load7(g, P, s, i, j, k0 - 2 + e, w);
+#pragma unroll
+      for (int v = 0; v < 7; v++) sv[v][e] = w[v];
+    }
   }
   __syncthreads();
   if (!pole && t < cnt + 2) {
@@ -924,21 +997,21 @@ __global__ void monopole_profile3_kernel(const ProbTime *__restrict__ times, Gri
 // second stage, the zone terms of the next estimate_dt (step.c:177-187).
 template <int STAGE>
 __global__ void __launch_bounds__(NT3, MDG_P3MINB) push3_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
-                                                     Grid3 g, const Tile3 *__restrict__ tiles, StateSoA sst,
+                                                     Grid3 g, StateSoA sst,
                                                      StateSoA sn, StateSoA out, const double *__restrict__ F0,
                                                      const double *__restrict__ F1, const double *__restrict__ F2)
 {
   __shared__ double sred[32];
+  __shared__ int sbeg[NT3];
   if (times[0].done) return;
   const ProbDev &P = probs[0];
   const double dt = times[0].dt;
-  const Tile3 t = tiles[blockIdx.x];
-  const int i = t.i, j = t.j, k = t.k0 + (int)threadIdx.x;
+  const int64_t c = (int64_t)blockIdx.x * NT3 + threadIdx.x;
+  const int row = zone_row(g, sbeg);
   double lmin = 1.0e300, lmax = 0.0;
-  if ((int)threadIdx.x < t.cnt) {
-    const int ij = rowi(g, i, j);
-    const PushRow3 &pr = g.prow[ij];
-    const int64_t c = pr.cell + k;
+  if (c < g.ncell) {
+    const PushRow3 &pr = g.prow[row];
+    const int i = pr.i, j = pr.j, ij = pr.ij, k = (int)(c - __ldg(g.rowcell + row));
     double ph[NPRIM], pn[NPRIM], u[NPRIM], uh[NPRIM], src[NPRIM], divF[NPRIM], pf[NPRIM];
 #pragma unroll
     for (int v = 0; v < NPRIM; v++) ph[v] = sst.v[v][c];
@@ -1081,17 +1154,17 @@ __global__ void __launch_bounds__(NT3, MDG_P3MINB) push3_kernel(const ProbDev *_
 
 // First estimate_dt of the problem (step.c:171-187, the EOS of the state itself).
 __global__ void __launch_bounds__(NT3) estimate3_kernel(const ProbDev *__restrict__ probs,
-                                                         ProbTime *__restrict__ times, Grid3 g,
-                                                         const Tile3 *__restrict__ tiles, StateSoA s)
+                                                         ProbTime *__restrict__ times, Grid3 g, StateSoA s)
 {
   __shared__ double sred[32];
+  __shared__ int sbeg[NT3];
   const ProbDev &P = probs[0];
-  const Tile3 t = tiles[blockIdx.x];
-  const int i = t.i, j = t.j, k = t.k0 + (int)threadIdx.x;
+  const int64_t c = (int64_t)blockIdx.x * NT3 + threadIdx.x;
+  const int row = zone_row(g, sbeg);
   double lmin = 1.0e300;
-  if ((int)threadIdx.x < t.cnt) {
-    const int ij = rowi(g, i, j);
-    const int64_t c = __ldg(g.cell + ij) + k;
+  if (c < g.ncell) {
+    const PushRow3 &pr = g.prow[row];
+    const int i = pr.i, j = pr.j, ij = pr.ij;
     const double rho = s.v[RHO][c], uu = s.v[UU][c];
     const double cs = sqrt(P.gam * eos_press(P.eos, P.gam, P.Kpoly, rho, uu) / rho);
     double local_dt = 0.0;
@@ -1161,15 +1234,22 @@ struct Sweep3 {
   char *d_tab = nullptr;           // all grid tables in one allocation
   double *d_flux = nullptr;        // F0 | F1 | F2, 5 arrays each
   unsigned char *d_bits = nullptr; // own0 | own1 | all0, one byte per zone each
-  Tile3 *d_tiles = nullptr;        // face2 | zone tiles
-  Tile3R *d_runs = nullptr;        // direction-0 face runs | direction-1 face runs
-  size_t runs_cap = 0;             // Tile3R entries d_runs holds
+  Tile3 *d_tiles = nullptr;        // zone tiles (the conserved totals)
+  int *d_seg = nullptr;            // direction-2 segments, then the first segment of every CTA
+  int nseg = 0;
+  int *d_row0 = nullptr;           // Grid3::row0
+  int *d_runs = nullptr;           // runs | runs | first run of every CTA | the same of direction 1
+  size_t runs_cap = 0;             // ints d_runs holds
+  size_t run_off[4] = {0, 0, 0, 0};
+  int nrun[2] = {0, 0}, nlane[2] = {0, 0};
   int run_len = RUN0;
+  int num_sms = 0;
   // the row structure the run lists are cut from (a copy of the host grid's)
   int n1 = 0, n2 = 0, n3 = 0;
   std::vector<int> nj, rowbase, nk;
   double *d_gmono = nullptr;       // monopole gravity per radial row
-  int nt[4] = {0, 0, 0, 0};
+  int nt[4] = {0, 0, 0, 0};        // CTAs of face0, face1, face2 and the zone kernels
+  int ntot = 0;                    // zone tiles of the conserved totals
   int64_t ncell = 0;
   int64_t bytes = 0;               // device memory held
 };
@@ -1179,72 +1259,167 @@ static void tiles_of_rows(std::vector<Tile3> &out, int i, int j, int count, int 
   for (int k0 = 0; k0 < count; k0 += chunk) out.push_back(Tile3{i, j, k0, (count - k0 < chunk) ? count - k0 : chunk});
 }
 
-// Work lists of the radial and theta run kernels for runs of at most run_len faces.
-static void build_runs(const Sweep3 &w, int run_len, std::vector<Tile3R> &t0, std::vector<Tile3R> &t1)
+// A run list: the runs, the run of each CTA's first lane, and the number of lanes.
+struct RunList {
+  std::vector<Run3> runs;
+  std::vector<int> first;
+  int nlane = 0;
+};
+
+// The faces of the radial (dir 0) or theta (dir 1) run kernel as runs of at most run_len
+// faces; cnt[r] is the number of columns of run r, k0[r] the first.
+static void cut_runs(const Sweep3 &w, int dir, int run_len, std::vector<Run3> &runs, std::vector<int> &cnt)
 {
   auto njr = [&](int i) { return w.nj[i + NG]; };
   auto row = [&](int i, int j) { return w.rowbase[i + NG] + j + NG; };
   auto dj = [&](int i) { return w.n2 / w.nj[i + NG]; };
   auto dk = [&](int i, int j) { return w.n3 / w.nk[row(i, j)]; };
-  t0.clear();
-  t1.clear();
-  // direction-0 runs: faces i in [0, n1] grouped by constant theta resolution, then per
-  // theta row j by constant phi resolution, cut into run_len faces and NT3 phi columns
-  for (int i = 0; i <= w.n1;) {
-    int ie = i + 1;
-    while (ie <= w.n1 && dj(ie) == dj(i)) ie++;
-    for (int j = 0; j < njr(i); j++) {
-      for (int a = i; a < ie;) {
+  if (dir == 0) {
+    // faces i in [0, n1] grouped by constant theta resolution, then per theta row j by
+    // constant phi resolution, cut into run_len faces
+    for (int i = 0; i <= w.n1;) {
+      int ie = i + 1;
+      while (ie <= w.n1 && dj(ie) == dj(i)) ie++;
+      for (int j = 0; j < njr(i); j++) {
+        for (int a = i; a < ie;) {
+          int b = a + 1;
+          while (b < ie && dk(b, j) == dk(a, j)) b++;
+          for (int c = a; c < b; c += run_len) {
+            runs.push_back(Run3{c, std::min(run_len, b - c), j, 0});
+            cnt.push_back(w.nk[row(a, j)]);
+          }
+          a = b;
+        }
+      }
+      i = ie;
+    }
+  } else {
+    // faces j in [0, nj(i)] of radial row i grouped by constant phi resolution of the face,
+    // min(dk(i, j), dk(i, j-1)), cut into run_len faces
+    for (int i = 0; i < w.n1; i++) {
+      const int nj = njr(i);
+      auto mn = [&](int j) { return std::min(dk(i, j), dk(i, j - 1)); };
+      for (int a = 0; a <= nj;) {
         int b = a + 1;
-        while (b < ie && dk(b, j) == dk(a, j)) b++;
-        const int nk = w.nk[row(a, j)];
-        for (int c = a; c < b; c += run_len)
-          for (int k0 = 0; k0 < nk; k0 += NT3)
-            t0.push_back(Tile3R{c, std::min(run_len, b - c), j, k0, std::min(NT3, nk - k0)});
+        while (b <= nj && mn(b) == mn(a)) b++;
+        for (int c = a; c < b; c += run_len) {
+          runs.push_back(Run3{c, std::min(run_len, b - c), i, 0});
+          cnt.push_back(w.n3 / mn(a));
+        }
         a = b;
       }
     }
-    i = ie;
   }
-  // direction-1 runs: faces j in [0, nj(i)] of radial row i grouped by constant phi
-  // resolution of the face, min(dk(i, j), dk(i, j-1)), cut into run_len faces and NT3 columns
+}
+
+// Longest run, up to run_len faces, for which the grid's lanes still fill the chip (5 CTAs of
+// 128 lanes on every SM).  What a lane does once, three pencil entries and a reconstruction,
+// is about two faces' worth, so long runs pay where there are lanes enough: ms per step on a
+// B200 for runs of 1 / 4 / 8 / 16, 2-D 400 x 256 mixed 0.206 / 0.287 / 0.419 / 0.712 (taken: 1),
+// 3-D 100 x 32 x 64 plain FP64 0.581 / 0.693 / 0.856 / 1.287 (1), 128 x 64 x 128 plain FP64 1.971 /
+// 1.802 / 1.695 / 2.179 (8), 384 x 128 x 256 plain FP64 11.55 / 9.07 / 8.60 / 8.46 (16).
+static int fitting_run(const Sweep3 &w, int run_len)
+{
+  const int64_t fill = (int64_t)(w.num_sms > 0 ? w.num_sms : 148) * 5 * NT3;
+  while (run_len > 1 && w.ncell / run_len < fill) run_len = (run_len + 1) / 2;
+  return run_len;
+}
+
+static void build_runs(const Sweep3 &w, int dir, int run_len, RunList &out)
+{
+  std::vector<Run3> runs;
+  std::vector<int> cnt;
+  cut_runs(w, dir, fitting_run(w, run_len), runs, cnt);
+  // long runs first (the tail of the launch is made of short ones), neighbouring rows in
+  // neighbouring lanes: direction 0 by first face then theta row, direction 1 likewise
+  std::vector<int> ord(runs.size());
+  for (size_t q = 0; q < ord.size(); q++) ord[q] = (int)q;
+  std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+    if (runs[a].nr != runs[b].nr) return runs[a].nr > runs[b].nr;
+    if (runs[a].r0 != runs[b].r0) return runs[a].r0 < runs[b].r0;
+    return runs[a].row < runs[b].row;
+  });
+  for (int q : ord) {
+    Run3 r = runs[q];
+    r.l0 = out.nlane;
+    out.nlane += cnt[q];
+    while ((int)out.first.size() * NT3 < out.nlane) out.first.push_back((int)out.runs.size());
+    out.runs.push_back(r);
+  }
+}
+
+// Direction-2 segments and the first segment of every CTA.
+static void build_segs(const Sweep3 &w, std::vector<Seg2> &segs, std::vector<int> &first)
+{
+  int used = 0, n = 0;   // lanes and segments of the CTA being filled
   for (int i = 0; i < w.n1; i++) {
-    const int nj = njr(i);
-    auto mn = [&](int j) { return std::min(dk(i, j), dk(i, j - 1)); };
-    for (int a = 0; a <= nj;) {
-      int b = a + 1;
-      while (b <= nj && mn(b) == mn(a)) b++;
-      const int cnt = w.n3 / mn(a);
-      for (int c = a; c < b; c += run_len)
-        for (int k0 = 0; k0 < cnt; k0 += NT3)
-          t1.push_back(Tile3R{c, std::min(run_len, b - c), i, k0, std::min(NT3, cnt - k0)});
-      a = b;
+    for (int j = 0; j < w.nj[i + NG]; j++) {
+      const int nf = w.nk[w.rowbase[i + NG] + j + NG] + 1;
+      for (int k0 = 0; k0 < nf;) {
+        int cnt = std::min(nf - k0, T2);
+        if (n == SEG2_MAX) used = n = 0;
+        if (used + cnt + 2 > NT3) {
+          // does not fit: cut it (two more lanes) where at least 8 faces do, else a new CTA
+          const int room = NT3 - used - 2;
+          if (room >= 8) cnt = room;
+          else used = n = 0;
+        }
+        if (n == 0) first.push_back((int)segs.size());
+        segs.push_back(Seg2{i, j, k0, cnt, used, n});
+        used += cnt + 2;
+        n++;
+        k0 += cnt;
+      }
     }
   }
+}
+
+// Both run lists for runs of at most run_len faces, into one device allocation.
+static cudaError_t upload_runs(Sweep3 *w, int run_len)
+{
+  RunList l[2];
+  std::vector<int> all;
+  size_t off[4];
+  for (int d = 0; d < 2; d++) {
+    build_runs(*w, d, run_len, l[d]);
+    off[d] = all.size();
+    const int *r = reinterpret_cast<const int *>(l[d].runs.data());
+    all.insert(all.end(), r, r + sizeof(Run3) / sizeof(int) * l[d].runs.size());
+  }
+  for (int d = 0; d < 2; d++) {
+    off[2 + d] = all.size();
+    all.insert(all.end(), l[d].first.begin(), l[d].first.end());
+  }
+  cudaError_t e = cudaSuccess;
+  if (all.size() > w->runs_cap) {
+    int *d = nullptr;
+    e = cudaMalloc(&d, sizeof(int) * all.size());
+    if (e != cudaSuccess) return e;
+    cudaFree(w->d_runs);
+    w->d_runs = d;
+    w->runs_cap = all.size();
+  }
+  e = cudaMemcpy(w->d_runs, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return e;
+  for (int q = 0; q < 4; q++) w->run_off[q] = off[q];
+  for (int d = 0; d < 2; d++) {
+    w->nt[d] = (int)l[d].first.size();
+    w->nrun[d] = (int)l[d].runs.size();
+    w->nlane[d] = l[d].nlane;
+  }
+  w->run_len = run_len;
+  return cudaSuccess;
 }
 
 int sweep3_set_run_length(Sweep3 *w, int run_length, std::string &why)
 {
   if (run_length < 1 || run_length > 64) { why = "run_length out of [1, 64]"; return MDG_ERR_INVALID; }
   if (run_length == w->run_len) return MDG_OK;
-  std::vector<Tile3R> t0, t1;
-  build_runs(*w, run_length, t0, t1);
-  const int n0 = (int)t0.size(), n1 = (int)t1.size();
-  t0.insert(t0.end(), t1.begin(), t1.end());
-  cudaError_t e = cudaSuccess;
-  if (t0.size() > w->runs_cap) {
-    Tile3R *d = nullptr;
-    e = cudaMalloc(&d, sizeof(Tile3R) * t0.size());
-    if (e != cudaSuccess) { why = cudaGetErrorString(e); return MDG_ERR_OUTOFMEM; }
-    cudaFree(w->d_runs);
-    w->d_runs = d;
-    w->runs_cap = t0.size();
+  const cudaError_t e = upload_runs(w, run_length);
+  if (e != cudaSuccess) {
+    why = cudaGetErrorString(e);
+    return e == cudaErrorMemoryAllocation ? MDG_ERR_OUTOFMEM : MDG_ERR_CUDA;
   }
-  e = cudaMemcpy(w->d_runs, t0.data(), sizeof(Tile3R) * t0.size(), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) { why = cudaGetErrorString(e); return MDG_ERR_CUDA; }
-  w->nt[0] = n0;
-  w->nt[1] = n1;
-  w->run_len = run_length;
   return MDG_OK;
 }
 
@@ -1256,8 +1431,11 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   if (h.nlev1 > G3_MAXLEV || h.nlev2 > G3_MAXLEV) { why = "too many refinement levels"; return MDG_ERR_INVALID; }
   Sweep3 *w = new Sweep3();
   w->ncell = h.ncell;
-  // push() flux addresses of every interior row (the fan-in rules of push3_kernel)
-  std::vector<PushRow3> prow((size_t)h.nij);
+  // push() flux addresses of every interior row (the fan-in rules of push3_kernel), in zone
+  // order, with the first zone of each row and the row of each CTA's first zone
+  std::vector<PushRow3> prow;
+  std::vector<int64_t> rowcell;
+  std::vector<int> row0;
   for (int i = 0; i < h.n1; i++) {
     for (int j = 0; j < h.njr(i); j++) {
       PushRow3 r{};
@@ -1276,8 +1454,12 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
       r.mo = (dkp > dkij) ? 1 : (dkp < dkij ? 2 : 0);
       r.mi = (dkm < dkij) ? 1 : 0;
       r.f2 = h.ndim == 3 ? h.f2[ij] : 0;
-      r.cell = h.cell[ij];
-      prow[ij] = r;
+      r.i = i;
+      r.j = j;
+      r.ij = ij;
+      while ((int64_t)row0.size() * NT3 < h.cell[ij] + h.nk[ij]) row0.push_back((int)prow.size());
+      prow.push_back(r);
+      rowcell.push_back(h.cell[ij]);
     }
   }
   // one allocation for every table, each part 256-byte aligned
@@ -1293,7 +1475,8 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
       {h.cphc.data(), h.cphc.size() * sizeof(double)},  {h.sphl.data(), h.sphl.size() * sizeof(double)},
       {h.cphl.data(), h.cphl.size() * sizeof(double)},  {h.mx0.data(), h.mx0.size() * sizeof(float)},
       {h.mx1.data(), h.mx1.size() * sizeof(float)},     {h.mx2.data(), h.mx2.size() * sizeof(float)},
-      {h.medge.data(), h.medge.size() * sizeof(double)},    {prow.data(), prow.size() * sizeof(PushRow3)}};
+      {h.medge.data(), h.medge.size() * sizeof(double)},    {prow.data(), prow.size() * sizeof(PushRow3)},
+      {rowcell.data(), rowcell.size() * sizeof(int64_t)}};
   std::vector<size_t> off(parts.size());
   size_t tot = 0;
   for (size_t q = 0; q < parts.size(); q++) {
@@ -1307,7 +1490,7 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   auto fail3 = [&](cudaError_t e) {
     why = cudaGetErrorString(e);
     cudaFree(w->d_tab); cudaFree(w->d_flux); cudaFree(w->d_bits); cudaFree(w->d_tiles); cudaFree(w->d_gmono);
-    cudaFree(w->d_runs);
+    cudaFree(w->d_runs); cudaFree(w->d_seg); cudaFree(w->d_row0);
     delete w;
     return e == cudaErrorMemoryAllocation ? MDG_ERR_OUTOFMEM : MDG_ERR_CUDA;
   };
@@ -1337,6 +1520,8 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   g.mx0 = (const float *)(b + off[19]); g.mx1 = (const float *)(b + off[20]); g.mx2 = (const float *)(b + off[21]);
   g.medge = (const double *)(b + off[22]);
   g.prow = (const PushRow3 *)(b + off[23]);
+  g.rowcell = (const int64_t *)(b + off[24]);
+  g.nrow = (int)prow.size();
   g.x0 = d.startx[0];
   g.mono = d.monopole;
   e = cudaMalloc(&w->d_gmono, sizeof(double) * (size_t)h.n1);
@@ -1350,28 +1535,41 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   e = cudaMemset(w->d_bits, 0, (size_t)3 * h.ncell);
   if (e != cudaSuccess) return fail3(e);
   // tiles of each kernel
-  std::vector<Tile3> t2, tc;
-  std::vector<Tile3R> t0, t1;
+  std::vector<Tile3> tc;
   w->n1 = h.n1; w->n2 = h.n2; w->n3 = h.n3;
   w->nj = h.nj; w->rowbase = h.rowbase; w->nk = h.nk;
-  build_runs(*w, RUN0, t0, t1);
-  for (int i = 0; i < h.n1 && h.ndim == 3; i++)
-    for (int j = 0; j < h.njr(i); j++) tiles_of_rows(t2, i, j, h.nk[h.row(i, j)] + 1, T2);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&w->num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    w->num_sms = 0;
   for (int i = 0; i < h.n1; i++)
     for (int j = 0; j < h.njr(i); j++) tiles_of_rows(tc, i, j, h.nk[h.row(i, j)]);
-  w->nt[0] = (int)t0.size(); w->nt[1] = (int)t1.size(); w->nt[2] = (int)t2.size(); w->nt[3] = (int)tc.size();
-  std::vector<Tile3> all;
-  all.insert(all.end(), t2.begin(), t2.end());
-  all.insert(all.end(), tc.begin(), tc.end());
-  e = cudaMalloc(&w->d_tiles, sizeof(Tile3) * all.size());
+  w->ntot = (int)tc.size();
+  w->nt[3] = (int)row0.size();
+  e = cudaMalloc(&w->d_row0, sizeof(int) * row0.size());
   if (e != cudaSuccess) return fail3(e);
-  e = cudaMemcpy(w->d_tiles, all.data(), sizeof(Tile3) * all.size(), cudaMemcpyHostToDevice);
+  e = cudaMemcpy(w->d_row0, row0.data(), sizeof(int) * row0.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail3(e);
-  t0.insert(t0.end(), t1.begin(), t1.end());
-  e = cudaMalloc(&w->d_runs, sizeof(Tile3R) * t0.size());
+  g.row0 = w->d_row0;
+  e = cudaMalloc(&w->d_tiles, sizeof(Tile3) * tc.size());
   if (e != cudaSuccess) return fail3(e);
-  w->runs_cap = t0.size();
-  e = cudaMemcpy(w->d_runs, t0.data(), sizeof(Tile3R) * t0.size(), cudaMemcpyHostToDevice);
+  e = cudaMemcpy(w->d_tiles, tc.data(), sizeof(Tile3) * tc.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return fail3(e);
+  if (h.ndim == 3) {
+    std::vector<Seg2> segs;
+    std::vector<int> first, all;
+    build_segs(*w, segs, first);
+    w->nt[2] = (int)first.size();
+    w->nseg = (int)segs.size();
+    const int *q = reinterpret_cast<const int *>(segs.data());
+    all.assign(q, q + sizeof(Seg2) / sizeof(int) * segs.size());
+    all.insert(all.end(), first.begin(), first.end());
+    e = cudaMalloc(&w->d_seg, sizeof(int) * all.size());
+    if (e != cudaSuccess) return fail3(e);
+    e = cudaMemcpy(w->d_seg, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail3(e);
+  }
+  e = upload_runs(w, RUN0);
   if (e != cudaSuccess) return fail3(e);
   *out = w;
   return MDG_OK;
@@ -1381,7 +1579,7 @@ void sweep3_destroy(Sweep3 *w)
 {
   if (!w) return;
   cudaFree(w->d_tab); cudaFree(w->d_flux); cudaFree(w->d_bits); cudaFree(w->d_tiles); cudaFree(w->d_gmono);
-  cudaFree(w->d_runs);
+  cudaFree(w->d_runs); cudaFree(w->d_seg); cudaFree(w->d_row0);
   delete w;
 }
 
@@ -1395,8 +1593,11 @@ void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, Prob
   const Grid3 &g = w->g;
   double *F0 = w->d_flux, *F1 = F0 + NPRIM * g.nf0, *F2 = F1 + NPRIM * g.nf1;
   unsigned char *own = w->d_bits + (size_t)stage * g.ncell, *all0 = w->d_bits + (size_t)2 * g.ncell;
-  const Tile3R *t0 = w->d_runs, *t1 = t0 + w->nt[0];
-  const Tile3 *t2 = w->d_tiles, *tc = t2 + w->nt[2];
+  const Run3 *r0 = reinterpret_cast<const Run3 *>(w->d_runs + w->run_off[0]);
+  const Run3 *r1 = reinterpret_cast<const Run3 *>(w->d_runs + w->run_off[1]);
+  const int *l0 = w->d_runs + w->run_off[2], *l1 = w->d_runs + w->run_off[3];
+  const Seg2 *segs = reinterpret_cast<const Seg2 *>(w->d_seg);
+  const int *l2 = w->d_seg + sizeof(Seg2) / sizeof(int) * w->nseg;
   if (stage == 0) cudaMemsetAsync(all0, 0, (size_t)g.ncell, st);
   if (g.mono) {
     shell_mass3_kernel<<<(g.n1 + 127) / 128, 128, 0, st>>>(times, g, sst);
@@ -1405,9 +1606,12 @@ void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, Prob
   auto faces = [&](auto s0, auto mix) {
     constexpr int S = decltype(s0)::value;
     constexpr bool M = decltype(mix)::value;
-    face0_kernel<M><<<w->nt[0], NT3, 0, st>>>(probs, times, g, t0, sst, F0, own, all0, S);
-    face1_kernel<M><<<w->nt[1], NT3, 0, st>>>(probs, times, g, t1, sst, F1, own, all0, S);
-    if (w->nt[2] > 0) face2_kernel<S, M><<<w->nt[2], NT3, 0, st>>>(probs, times, g, t2, sst, F2, own, all0);
+    face0_kernel<M><<<w->nt[0], NT3, 0, st>>>(probs, times, g, r0, w->nrun[0], l0, w->nlane[0], sst, F0, own,
+                                                  all0, S);
+    face1_kernel<M><<<w->nt[1], NT3, 0, st>>>(probs, times, g, r1, w->nrun[1], l1, w->nlane[1], sst, F1, own,
+                                                  all0, S);
+    if (w->nt[2] > 0)
+      face2_kernel<S, M><<<w->nt[2], NT3, 0, st>>>(probs, times, g, segs, w->nseg, l2, sst, F2, own, all0);
   };
   using I0 = std::integral_constant<int, 0>;
   using I1 = std::integral_constant<int, 1>;
@@ -1415,23 +1619,21 @@ void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, Prob
   using BT = std::integral_constant<bool, true>;
   if (stage == 0) {
     if (mixed) faces(I0{}, BT{}); else faces(I0{}, BF{});
-    push3_kernel<0><<<w->nt[3], NT3, 0, st>>>(probs, times, g, tc, sst, sn, out, F0, F1, F2);
+    push3_kernel<0><<<w->nt[3], NT3, 0, st>>>(probs, times, g, sst, sn, out, F0, F1, F2);
   } else {
     if (mixed) faces(I1{}, BT{}); else faces(I1{}, BF{});
-    push3_kernel<1><<<w->nt[3], NT3, 0, st>>>(probs, times, g, tc, sst, sn, out, F0, F1, F2);
+    push3_kernel<1><<<w->nt[3], NT3, 0, st>>>(probs, times, g, sst, sn, out, F0, F1, F2);
   }
 }
 
 void launch_totals3(Sweep3 *w, StateSoA s, double *out, cudaStream_t st)
 {
-  const Tile3 *tc = w->d_tiles + w->nt[2];
-  totals3_kernel<<<1, 256, 0, st>>>(w->g, tc, w->nt[3], s, out);
+  totals3_kernel<<<1, 256, 0, st>>>(w->g, w->d_tiles, w->ntot, s, out);
 }
 
 void launch_initial_estimate3(Sweep3 *w, const ProbDev *probs, ProbTime *times, StateSoA s, cudaStream_t st)
 {
-  const Tile3 *tc = w->d_tiles + w->nt[2];
-  estimate3_kernel<<<w->nt[3], NT3, 0, st>>>(probs, times, w->g, tc, s);
+  estimate3_kernel<<<w->nt[3], NT3, 0, st>>>(probs, times, w->g, s);
 }
 
 }  // namespace mdg

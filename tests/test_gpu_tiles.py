@@ -1,11 +1,12 @@
 """Work lists of the sweeps at the sizes where they can go wrong: the rows per 2-D tile
-follow the grid size (tile_rows_2d, mdg_sweep2d.cu), so the results must not depend on where
-the tiles are cut.  Bars as in test_gpu_parity.py: <= 1e-12 per step."""
+follow the grid size (tile_rows_2d, mdg_sweep2d.cu), and the dendritic sweeps pack rows of 1 to 256 phi zones
+into CTAs and cut their runs by the grid size, so the results must not depend on where the
+cuts fall.  Bars as in test_gpu_parity.py: <= 1e-12 per step; run lengths bit for bit."""
 import numpy as np
 import pytest
 
 from medusa_b200 import problems as P
-from medusa_b200.solver import Solver
+from medusa_b200.solver import PREC_FP64, PREC_MIXED, Solver
 from oracle import pyoracle
 from tests._cases import field_rel_err, pointwise_rel_err
 
@@ -29,3 +30,21 @@ def test_2d_tile_edges_match_the_oracle(kind, n1, n2):
     assert np.all(np.isfinite(got))
     assert field_rel_err(got, ref) <= 1.0e-12 * steps
     assert pointwise_rel_err(got, ref, pb) <= 1.0e-12 * steps
+
+
+# 2-D rows of one phi zone (a last CTA with idle lanes), small 3-D rows several to a CTA, rows
+# of 128 phi zones (cut segments) on a grid whose runs the size rule leaves at 1, 8 and more
+@pytest.mark.parametrize("dims", [(71, 64, 1), (33, 16, 32), (60, 64, 128), (220, 64, 128)])
+@pytest.mark.parametrize("prec", [PREC_FP64, PREC_MIXED])
+def test_dendritic_work_lists_do_not_change_the_results(dims, prec):
+    n1, n2, n3 = dims
+    pb = P.sedov_2d_spherical(n1, n2, noise=0.01) if n3 == 1 else P.sedov_3d(n1, n2, n3, noise=0.01)
+    out = []
+    for run in (1, 3, 64):
+        with Solver(pb, precision=prec) as s:
+            s.set_launch_config(run_length=run)
+            s.step(2)
+            s.synchronize()
+            out.append(s.update_cpu(0))
+    assert np.all(np.isfinite(out[0]))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
