@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include "mdg_internal.h"
+#include "mdg_recon.h"
 
 namespace mdg {
 
@@ -33,58 +34,6 @@ struct RcView {
   }
 };
 
-// para_recon for one zone (reconstruct.c:142-201): am/a0/ap are the zone averages at
-// i-1, i, i+1; returns the left (al) and right (ar) face values of zone i.
-//
-// Control flow is arranged for the SIMT machine without changing any result: the
-// extremum test (reconstruct.c:145) only skips the work when every active lane of the
-// warp is at an extremum; otherwise all lanes compute and extremum lanes select a[i] at
-// the end, so the six variables of a zone run as independent instruction streams.  The
-// two "move the zero" cases (reconstruct.c:190-200) share one code path.
-template <typename T, typename G>
-__device__ __forceinline__ void para_recon_zone(T am_v, T a, T ap_v, const G &g, T &al, T &ar)
-{
-  T dqm = a - am_v;
-  T dqp = ap_v - a;
-  const bool flat = (dqm * dqp <= T(0));
-  if (__all_sync(__activemask(), flat)) { al = a; ar = a; return; }
-  T dqc = ap_v - am_v;
-  T A = (dqm * g(RC_BP) * g(RC_GM) * g(RC_G0) + g(RC_GP) * (dqp * g(RC_BM) * g(RC_G0) - dqc * g(RC_B0) * g(RC_GM))) * g(RC_DEN1);
-  T B = -(dqm * g(RC_AP) * g(RC_GM) * g(RC_G0) + g(RC_GP) * (dqp * g(RC_AM) * g(RC_G0) - dqc * g(RC_A0) * g(RC_GM))) * g(RC_DEN1);
-  T C = a - (g(RC_A0) * A + g(RC_B0) * B) / g(RC_G0);
-  const T xl = g(RC_XL), xr = g(RC_XR);
-  T l = xl * (A * xl + B) + C;
-  T r = xr * (A * xr + B) + C;
-  T mean = T(0.75) * am_v + T(0.25) * a;
-  T mask = (a - l) * (l - mean);
-  l = (mask < T(0)) ? mean : l;
-  mean = T(0.75) * ap_v + T(0.25) * a;
-  mask = (mean - r) * (r - a);
-  r = (mask < T(0)) ? mean : r;
-  A = (g(RC_B0) * (r - l) + g(RC_G0) * (a * g(RC_XLR) - r * xl + l * xr)) * g(RC_DEN2);
-  B = (g(RC_A0) * (l - r) + g(RC_G0) * (r - a) * g(RC_XL2) + g(RC_G0) * (a - l) * g(RC_XR2)) * g(RC_DEN2);
-  T xzero = -B / (T(2) * A + T(1.0e-16));
-  if (isinf(xzero) || isnan(xzero)) xzero = T(-1.0e-200);
-  const bool inside = !flat && (xzero > xl && xzero < xr);
-  if (__any_sync(__activemask(), inside)) {
-    // move the zero to the right edge (replace al) or to the left edge (replace ar)
-    const bool right = xzero > g(RC_XMID);
-    const T e = right ? r : l;
-    const T xe = right ? xr : xl;
-    const T xo = right ? xl : xr;
-    A = g(RC_G0) * (a - e) / (right ? g(RC_DMR) : g(RC_DML));
-    B = T(-2.0) * A * xe;
-    C = a - (g(RC_A0) * A + g(RC_B0) * B) / g(RC_G0);
-    const T val = xo * (A * xo + B) + C;
-    if (inside) {
-      if (right) l = val;
-      else r = val;
-    }
-  }
-  al = flat ? a : l;
-  ar = flat ? a : r;
-}
-
 // lin_recon for one zone (reconstruct.c:99-121)
 template <typename T, typename G>
 __device__ __forceinline__ void lin_recon_zone(T am_v, T a, T ap_v, const G &g, T &al, T &ar)
@@ -99,43 +48,35 @@ __device__ __forceinline__ void lin_recon_zone(T am_v, T a, T ap_v, const G &g, 
   ar = A * g(RC_XR) + B;
 }
 
-// How the FP64 reconstruction is emitted, chosen per translation unit before this header
-// is included (the results are the same either way):
-//   MDG_RECON_OUTLINE 1 -- recon_zone calls one out-of-line copy of para_recon/lin_recon
-//                          (kernels whose many inlined copies overflow the instruction
-//                          cache: the 1-D stage and the 3-D face kernels);
-//   MDG_RECON_UNROLL n  -- unroll factor of the loops over the reconstructed variables
-//                          (1: one inlined copy per loop, the 2-D split sweep).
-#ifndef MDG_RECON_OUTLINE
-#define MDG_RECON_OUTLINE 0
-#endif
-#ifndef MDG_RECON_UNROLL
-#define MDG_RECON_UNROLL 8
-#endif
-constexpr int kReconUnroll = MDG_RECON_UNROLL;
 struct FacePair { double al, ar; };
 template <typename G>
-__device__ __noinline__ FacePair recon_zone_call(int order, double am_v, double a, double ap_v, G g)
+__device__ __noinline__ FacePair recon_declined(double am, double a, double ap, G g)
 {
   FacePair o;
-  if (order == 3) para_recon_zone(am_v, a, ap_v, g, o.al, o.ar);
-  else if (order == 2) lin_recon_zone(am_v, a, ap_v, g, o.al, o.ar);
-  else { o.al = a; o.ar = a; }
+  para_recon_zone<double>(am, a, ap, g, o.al, o.ar);
   return o;
 }
 
-template <typename T, typename G>
-__device__ __forceinline__ void recon_zone(int order, T am_v, T a, T ap_v, const G &g, T &al, T &ar)
+// NV variables of one zone in order `order`: at(v, q) is variable v's average in zone i-1+q,
+// put(v, al, ar) takes its face values.  The loop is not unrolled: one copy of the code per
+// loop keeps the kernels in the instruction cache.
+template <int NV, typename G, typename At, typename Put>
+__device__ __forceinline__ void recon_vars(int order, const G &g, At at, Put put)
 {
-  if (MDG_RECON_OUTLINE && sizeof(T) == 8) {
-    const FacePair o = recon_zone_call<G>(order, am_v, a, ap_v, g);
-    al = o.al;
-    ar = o.ar;
-    return;
+#pragma unroll 1
+  for (int v = 0; v < NV; v++) {
+    const double am = at(v, 0), a = at(v, 1), ap = at(v, 2);
+    FacePair o;
+    if (order == 3) {
+      if (!para_recon_fast(am, a, ap, g, o.al, o.ar)) o = recon_declined<G>(am, a, ap, g);
+    } else if (order == 2) {
+      lin_recon_zone(am, a, ap, g, o.al, o.ar);
+    } else {
+      o.al = a;
+      o.ar = a;
+    }
+    put(v, o.al, o.ar);
   }
-  if (order == 3) para_recon_zone(am_v, a, ap_v, g, al, ar);
-  else if (order == 2) lin_recon_zone(am_v, a, ap_v, g, al, ar);
-  else { al = a; ar = a; }
 }
 
 // Geometry of one face as the Riemann solver sees it (zone_geom at the face's cell).
@@ -175,6 +116,51 @@ __device__ __forceinline__ GamConst<T> gam_const(T G)
   return c;
 }
 
+// The two tests that the solvers make on a face's pressure ratio: (p_max - p_min) / p_min >
+// 0.5 (shock tag) and p_max / p_min < 2.  In FP64, for positive p_min, fl(x / y) > 0.5 exactly
+// when x > 0.5 y and fl(x / y) < 2 exactly when x < 2 y: the quotient of two numbers that
+// differ from the ratio 1/2 or 2 at all differs by more than the half ulp that rounding
+// could close.  (FP32 keeps its approximate quotients.)
+template <typename T>
+__device__ __forceinline__ void pressure_ratio_tests(T p_max, T p_min, bool &below2, int &isshock)
+{
+  if (sizeof(T) == 8 && p_min > T(0x1p-100) * T(0x1p-100) && p_max < T(0x1p120) * T(0x1p120)) {
+    below2 = p_max < T(2) * p_min;
+    isshock = (p_max - p_min > T(0.5) * p_min) ? 1 : 0;
+  } else {
+    below2 = p_max / p_min < T(2);
+    isshock = ((p_max - p_min) / p_min > T(0.5)) ? 1 : 0;
+  }
+}
+
+// q[v] = a[v] / b, correctly rounded, by one reciprocal (div_by): a zero numerator is its
+// own quotient for b > 0; numbers outside recon_in_range and b <= 0 take the division.
+// MIX (the mixed sweeps, whose results are not pinned to the reference's rounding): the
+// product with the reciprocal.
+template <int N>
+__device__ __noinline__ void quotients_declined(const double (&a)[N], double b, double (&q)[N])
+{
+  for (int v = 0; v < N; v++) q[v] = a[v] / b;
+}
+template <int N, bool MIX = false>
+__device__ __forceinline__ void quotients(const double (&a)[N], double b, double (&q)[N])
+{
+  const double y = 1.0 / b;
+  if (MIX) {
+#pragma unroll
+    for (int v = 0; v < N; v++) q[v] = a[v] * y;
+    return;
+  }
+  bool ok = b > 0.0 && recon_in_range(b);
+#pragma unroll
+  for (int v = 0; v < N; v++) {
+    q[v] = div_by(a[v], b, y);
+    q[v] = (a[v] == 0.0) ? a[v] : q[v];
+    ok = ok && (a[v] == 0.0 || recon_in_range(a[v]));
+  }
+  if (!ok) quotients_declined<N>(a, b, q);
+}
+
 // Wave-speed estimate shared by HLLC and HLLE (riemann.c:368-429 / 210-303).
 // w[0..4] primitives, w[5] pressure (w[6], Gamma, equals gc.g).
 template <typename T>
@@ -186,13 +172,13 @@ __device__ __forceinline__ void wave_speeds(const T *pl, const T *pr, T u_l, T u
   T cs_r = sqrt(G * p_r / pr[RHO]);
   T p_max, p_min;
   if (p_l > p_r) { p_max = p_l; p_min = p_r; } else { p_max = p_r; p_min = p_l; }
-  T pratio = p_max / p_min;
-  isshock = ((p_max - p_min) / p_min > T(0.5)) ? 1 : 0;
+  bool below2;
+  pressure_ratio_tests(p_max, p_min, below2, isshock);
   p_s = T(0.5) * (p_l + p_r) - T(0.125) * (u_r - u_l) * (pl[RHO] + pr[RHO]) * (cs_l + cs_r);
   // HLLC clamps with MAX(0,p_s), HLLE with MAX(p_s,0.0): they differ only for NaN
   if (hlle) p_s = (p_s > T(0)) ? p_s : T(0);
   else p_s = (T(0) > p_s) ? T(0) : p_s;
-  if (pratio < T(2) && p_s >= p_min && p_s <= p_max) {
+  if (below2 && p_s >= p_min && p_s <= p_max) {
     // primitive-variable estimate kept
   } else if (p_s < p_min) {
     // two rarefactions (Toro 9.35-9.36)
@@ -345,11 +331,15 @@ __device__ __forceinline__ void p_to_u(const double *p, double *u, double g0, do
 // hydro_u_to_p (fluid.c:27-53); u is modified as in the reference.  With floors (the
 // ENFORCE_FLOORS build, fluid.c:43-46) density and internal energy are clamped from below
 // with the reference's MAX (decs.h:628) after the velocities are formed.
+template <bool MIX = false>
 __device__ __forceinline__ void u_to_p(double *u, double *p, double gc0, double gc1, double gc2,
                                        bool floors = false, double rho_floor = 0.0, double e_floor = 0.0)
 {
   p[RHO] = u[RHO];
-  u[U1] /= u[RHO]; u[U2] /= u[RHO]; u[U3] /= u[RHO];
+  const double mom[3] = {u[U1], u[U2], u[U3]};
+  double vel[3];
+  quotients<3, MIX>(mom, u[RHO], vel);
+  u[U1] = vel[0]; u[U2] = vel[1]; u[U3] = vel[2];
   p[U1] = gc0 * u[U1]; p[U2] = gc1 * u[U2]; p[U3] = gc2 * u[U3];
   double vsq = 0.0;
   vsq += u[U1] * p[U1]; vsq += u[U2] * p[U2]; vsq += u[U3] * p[U3];

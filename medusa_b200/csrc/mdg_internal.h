@@ -35,9 +35,8 @@ enum ReconField {
   RC_XL, RC_XR,               // x[i], x[i+1] (zone edges)
   RC_DEN1,                    // 1/(a0b1g2 + a1b2g0 + a2b0g1 - a0b2g1 - a1b0g2 - a2b1g0)
   RC_DEN2,                    // 1/((x[i]-x[i+1])*(alpha[i] + Gamma[i]x[i]x[i+1] - beta[i](x[i]+x[i+1])))
-  RC_XLR,                     // x[i]-x[i+1]
-  RC_XL2, RC_XR2,             // SQR(x[i]), SQR(x[i+1])
-  RC_XMID,                    // 0.5*(x[i]+x[i+1])
+  RC_RG0, RC_RDMR, RC_RDML,   // reciprocals of RC_G0, RC_DMR, RC_DML
+  RC_XEPS,                    // 2^-51 max(|x[i]|, |x[i+1]|); inf: para_recon_fast declines the zone
   RC_DMR, RC_DML,             // alpha + xhi*(Gamma*xhi - 2 beta), alpha + xlo*(Gamma*xlo - 2 beta)
   RC_LSM, RC_LSP, RC_LSC,     // lin_recon denominators x0-0.5(x[i]+xm), 0.5(x[i+1]+xp)-x0, xp-xm
   RC_NFIELDS

@@ -18,10 +18,6 @@
 // sequence of many steps in one launch -- the dt rules, both RK stages and the time
 // update, separated by cluster barriers -- where the per-phase path pays four dependent
 // launches per step.  It runs the same tile code, so the two paths agree bit for bit.
-// The FP64 reconstruction is called out of line here (one copy of para_recon in the
-// kernel instead of six): the kernel is bound by instruction fetch and load latency, and
-// the smaller code ran the 2048-problem ensemble 18 % faster on a B200 (same results).
-#define MDG_RECON_OUTLINE 1
 #include "mdg_hydro.cuh"
 #include "mdg_kernels.cuh"
 #include "mdg_load1d.cuh"
@@ -119,8 +115,8 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     int zc = z < -1 ? -1 : (z > n1 ? n1 : z);
     const int64_t c = P.geo_off + zc + NG;
     const RcView<double, !TMA> g{TMA ? &s_rc[0][c - bx] : rc + c, TMA ? (int64_t)TMA_COLS1 : rcs};
-#pragma unroll kReconUnroll
-    for (int v = 0; v < 6; v++) recon_zone<double>(P.interp_order, sv[v][t], sv[v][t + 1], sv[v][t + 2], g, al[v], ar[v]);
+    recon_vars<6>(P.interp_order, g, [&](int v, int q) { return sv[v][t + q]; },
+                  [&](int v, double lo, double hi) { al[v] = lo; ar[v] = hi; });
     al[6] = P.gam; ar[6] = P.gam;
   }
   if (TMA) __syncthreads();   // every zone reconstructed: the recon rows may be overwritten
@@ -194,9 +190,11 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     for (int v = 0; v < NPRIM; v++) { divF[v] = 0.0; divF[v] += sfl[v][t + 1]; divF[v] -= sfl[v][t]; }
     const double vol = gf(GF_VOL, gi);
     const double pfact = STAGE ? 0.5 : 1.0, phfact = STAGE ? 0.5 : 0.0, ffact = STAGE ? 0.5 : 1.0;
+    double dv[NPRIM];
+    quotients<NPRIM>(divF, vol, dv);
 #pragma unroll
     for (int v = 0; v < NPRIM; v++) {
-      double ddt = divF[v] / vol - src[v];
+      double ddt = dv[v] - src[v];
       u[v] = pfact * u[v] + phfact * uh[v] - ffact * dt * ddt;
     }
     u_to_p(u, pf, gf(GF_GC0, gi), gf(GF_GC1, gi), gf(GF_GC2, gi), P.floors != 0, P.rho_floor, P.e_floor);

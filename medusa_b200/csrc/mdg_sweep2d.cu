@@ -36,12 +36,6 @@
 //
 // Cartesian metric: gcov = gcon = scale = 1, so the metric multiplications and divisions
 // (exact identities) are compiled out (UNIT = true).
-// The per-variable reconstruction loops are not unrolled here (one inlined copy of
-// para_recon per loop): 7.5 % faster on the 2048^2 Kelvin-Helmholtz grid on a B200 than
-// unrolled, and faster than an out-of-line call there (same results).
-#ifndef MDG_RECON_UNROLL
-#define MDG_RECON_UNROLL 1
-#endif
 #include "mdg_hydro.cuh"
 #include "mdg_kernels.cuh"
 #include "mdg_mixed.cuh"
@@ -127,13 +121,8 @@ __device__ __noinline__ void face2d_fp64(int order, const double (&a)[6][4], con
                                          const FaceGeom<double> &fg, double *f, double &sig)
 {
   double pl[7], pr[7];
-  for (int v = 0; v < 6; v++) {
-    double lo, hi;
-    recon_zone<double>(order, a[v][0], a[v][1], a[v][2], gm, lo, hi);
-    pl[v] = hi;
-    recon_zone<double>(order, a[v][1], a[v][2], a[v][3], gz, lo, hi);
-    pr[v] = lo;
-  }
+  recon_vars<6>(order, gm, [&](int v, int q) { return a[v][q]; }, [&](int v, double, double hi) { pl[v] = hi; });
+  recon_vars<6>(order, gz, [&](int v, int q) { return a[v][1 + q]; }, [&](int v, double lo, double) { pr[v] = lo; });
   pl[6] = gam;
   pr[6] = gam;
   riemann_hllc<DIR, true, double>(pl, pr, fg, gam_const(gam), f, sig);
@@ -144,7 +133,7 @@ __device__ __noinline__ void face2d_fp64(int order, const double (&a)[6][4], con
 // accumulation, update and dt); faces the FP32 solver declines are re-solved in FP64,
 // which needs the zone before the face's left zone: the column ring keeps 5 rows.
 template <int STAGE, bool MIX>
-__global__ void __launch_bounds__(NTX2, MDG_XMINB)
+__global__ void __launch_bounds__(NTX2, MIX ? MDG_MIX2_MINB : MDG_XMINB)
 xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                 const Tile *__restrict__ tiles, Tables tb, StateSoA sst, StateSoA acc,
                 unsigned char *__restrict__ shock)
@@ -241,10 +230,8 @@ xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
         xl[6] = P.gam;
       } else {
         const RcView<double, false> g{&xrc[0][r - i0 + 1], TIX2 + 2};
-#pragma unroll kReconUnroll
-        for (int v = 0; v < 6; v++)
-          recon_zone<double>(order, ring[slot(r - 1)][v][t], ring[slot(r)][v][t], ring[slot(r + 1)][v][t], g,
-                             xl[v], xr[v]);
+        recon_vars<6>(order, g, [&](int v, int q) { return ring[slot(r - 1 + q)][v][t]; },
+                      [&](int v, double al, double ar) { xl[v] = al; xr[v] = ar; });
         xl[6] = P.gam;
       }
       if (r >= i0) {
@@ -295,7 +282,7 @@ xsweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
 
 // ------------------------------------------------------------------ direction 1 + push
 template <int STAGE, bool MIX>
-__global__ void __launch_bounds__(NTY2, MDG_YMINB)
+__global__ void __launch_bounds__(NTY2, MIX ? MDG_MIX2_MINB : MDG_YMINB)
 ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                 const Tile *__restrict__ tiles, Tables tb, StateSoA sst, StateSoA sn, StateSoA acc,
                 StateSoA out, const unsigned char *__restrict__ shock0, const unsigned char *__restrict__ shock1)
@@ -392,11 +379,8 @@ ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
       yl[6] = gam;
     } else {
       const RcView<double, false> g{&yrc[0][t], NTY2};
-      double yr[6];
-#pragma unroll kReconUnroll
-      for (int v = 0; v < 6; v++) recon_zone<double>(order, sv[v][t], sv[v][t + 1], sv[v][t + 2], g, yl[v], yr[v]);
-#pragma unroll
-      for (int v = 0; v < 6; v++) syr[v][t] = yr[v];
+      recon_vars<6>(order, g, [&](int v, int q) { return sv[v][t + q]; },
+                    [&](int v, double al, double ar) { yl[v] = al; syr[v][t] = ar; });
       yl[6] = gam;
     }
     __syncthreads();
@@ -449,15 +433,20 @@ ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
         nmin = tmin(nmin, src_dt_numerator_min(pn, u));   // dt_source_control, step.c:393
       }
       const double pfact = STAGE ? 0.5 : 1.0, phfact = STAGE ? 0.5 : 0.0, ffact = STAGE ? 0.5 : 1.0;
+      double divF[NPRIM], dv[NPRIM];
 #pragma unroll
       for (int v = 0; v < NPRIM; v++) {
-        double divF = accv[v];
-        divF += sfy[v][t + 1];
-        divF -= sfy[v][t];
-        double ddt = divF / P.vol - src[v];
+        divF[v] = accv[v];
+        divF[v] += sfy[v][t + 1];
+        divF[v] -= sfy[v][t];
+      }
+      quotients<NPRIM, MIX>(divF, P.vol, dv);
+#pragma unroll
+      for (int v = 0; v < NPRIM; v++) {
+        double ddt = dv[v] - src[v];
         u[v] = pfact * u[v] + phfact * uh[v] - ffact * dt * ddt;
       }
-      u_to_p(u, pf, 1.0, 1.0, 1.0, P.floors != 0, P.rho_floor, P.e_floor);
+      u_to_p<MIX>(u, pf, 1.0, 1.0, 1.0, P.floors != 0, P.rho_floor, P.e_floor);
 #pragma unroll
       for (int v = 0; v < NPRIM; v++) out.v[v][cell] = pf[v];
       flag_nonfinite(pf, &times[tile.prob]);

@@ -29,11 +29,6 @@
 //  * the polar-axis fix (step.c:1301-1401): on the last theta row of every radial row
 //    the phi-face states are the zone values with the velocity rotated through
 //    Cartesian components (host tables of the sines and cosines).
-// The FP64 reconstruction is called out of line here (face kernels would otherwise hold
-// 14 inlined copies of para_recon): instruction-fetch stalls were the largest stall of
-// the face kernels, and the smaller code ran the 384 x 128 x 256 Sedov grid 20 % faster
-// on a B200 (same results).
-#define MDG_RECON_OUTLINE 1
 #include "mdg_hydro.cuh"
 #include "mdg_kernels.cuh"
 #include "mdg_grid3d.cuh"
@@ -48,12 +43,18 @@ namespace mdg {
 
 struct Tile3 { int i, j, k0, cnt; };
 constexpr int NT3 = 128;
-// resident CTAs per SM requested from the compiler (register caps): the face kernels
-// wait on dependent gathers, and 8 CTAs of 4 warps (64 registers, a few spills) ran
-// 1.2x faster than 4 CTAs (128 registers) on the 384x128x256 Sedov grid
+// resident CTAs per SM requested from the compiler (register caps).  The face kernels wait
+// on dependent gathers and on FP64 latency; ms per step on a B200 with 8 / 6 / 5 / 4 CTAs of
+// 128 threads (64 / 80 / 96 / 128 registers): plain FP64 384 x 128 x 256 7.53 / 7.10 / 7.28 /
+// 7.84, 128 x 64 x 128 1.49 / 1.39 / 1.63 / 1.62; mixed 384 x 128 x 256 5.97 (8), 5.87 (7 and 6),
+// 6.07 (5), 6.55 (4).
 #ifndef MDG_F3MINB
-#define MDG_F3MINB 8
+#define MDG_F3MINB 6
 #endif
+#ifndef MDG_F3MINB_MIX
+#define MDG_F3MINB_MIX 7
+#endif
+constexpr int f3_minb(bool mix) { return mix ? MDG_F3MINB_MIX : MDG_F3MINB; }
 #ifndef MDG_P3MINB
 #define MDG_P3MINB 8
 #endif
@@ -293,12 +294,12 @@ __device__ __forceinline__ void wave_speeds_g(const double *pl, const double *pr
   const double cs_r = sqrt(G_r * p_r / pr[RHO]);
   double p_max, p_min;
   if (p_l > p_r) { p_max = p_l; p_min = p_r; } else { p_max = p_r; p_min = p_l; }
-  const double pratio = p_max / p_min;
-  isshock = ((p_max - p_min) / p_min > 0.5) ? 1 : 0;
+  bool below2;
+  pressure_ratio_tests(p_max, p_min, below2, isshock);
   p_s = 0.5 * (p_l + p_r) - 0.125 * (u_r - u_l) * (pl[RHO] + pr[RHO]) * (cs_l + cs_r);
   if (hlle) p_s = (p_s > 0.0) ? p_s : 0.0;
   else p_s = (0.0 > p_s) ? 0.0 : p_s;
-  if (pratio < 2.0 && p_s >= p_min && p_s <= p_max) {
+  if (below2 && p_s >= p_min && p_s <= p_max) {
   } else if (p_s < p_min) {
     const double G_avg = 0.5 * (G_l + G_r);
     const double plr = pow(p_l / p_r, (G_avg - 1.0) / (2.0 * G_avg));
@@ -408,14 +409,8 @@ __device__ __forceinline__ void recon_face(int order, const double pen[4][7], co
                                            int64_t c1, int64_t c2, double *pl, double *pr)
 {
   const RcView<double, true> g1{rc + c1, stride}, g2{rc + c2, stride};
-#pragma unroll kReconUnroll
-  for (int v = 0; v < 7; v++) {
-    double al, ar;
-    recon_zone<double>(order, pen[0][v], pen[1][v], pen[2][v], g1, al, ar);
-    pl[v] = ar;
-    recon_zone<double>(order, pen[1][v], pen[2][v], pen[3][v], g2, al, ar);
-    pr[v] = al;
-  }
+  recon_vars<7>(order, g1, [&](int v, int q) { return pen[q][v]; }, [&](int v, double, double hi) { pl[v] = hi; });
+  recon_vars<7>(order, g2, [&](int v, int q) { return pen[1 + q][v]; }, [&](int v, double lo, double) { pr[v] = lo; });
 }
 
 // Mixed precision (MIX): the same pencils, para_recon in FP32 difference form with the
@@ -553,7 +548,7 @@ __device__ __forceinline__ Run3 lane_run(const Run3 *__restrict__ runs, int nrun
 // face kernels): both stages then run the same code, which measured faster for stage 1
 // than its own specialisation.
 template <bool MIX>
-__global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face0_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Run3 *__restrict__ runs, int nrun,
                                                      const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, unsigned char *__restrict__ own,
@@ -596,12 +591,8 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *_
         }
       } else {
         const RcView<double, true> gz{g.rc0 + i0 - 1 + NG, rcs};
-#pragma unroll kReconUnroll
-        for (int v = 0; v < 7; v++) {
-          double al, ar;
-          recon_zone<double>(P.interp_order, win[sm][v][tid], win[s0][v][tid], win[sp][v][tid], gz, al, ar);
-          arb[v][tid] = ar;
-        }
+        recon_vars<7>(P.interp_order, gz, [&](int v, int q) { return win[q == 0 ? sm : q == 1 ? s0 : sp][v][tid]; },
+                      [&](int v, double, double hi) { arb[v][tid] = hi; });
       }
     }
 #pragma unroll 1
@@ -627,14 +618,8 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *_
         }
       } else {
         const RcView<double, true> gz{g.rc0 + i + NG, rcs};
-#pragma unroll kReconUnroll
-        for (int v = 0; v < 7; v++) {
-          pl[v] = arb[v][tid];
-          double al, ar;
-          recon_zone<double>(P.interp_order, win[sm][v][tid], win[s0][v][tid], win[sp][v][tid], gz, al, ar);
-          pr[v] = al;
-          arb[v][tid] = ar;
-        }
+        recon_vars<7>(P.interp_order, gz, [&](int v, int q) { return win[q == 0 ? sm : q == 1 ? s0 : sp][v][tid]; },
+                      [&](int v, double lo, double hi) { pl[v] = arb[v][tid]; pr[v] = lo; arb[v][tid] = hi; });
       }
       const int ij = rowi(g, i, j);
       const FaceGeom<double> fg = face_geom3<0>(g, ij);
@@ -687,7 +672,7 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face0_kernel(const ProbDev *_
 // column, one new entry and one zone reconstruction per face.  Run3 fields here:
 // r0 = j0, nr = faces, row = i.
 template <bool MIX>
-__global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face1_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Run3 *__restrict__ runs, int nrun,
                                                      const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
@@ -729,12 +714,8 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *_
         }
       } else {
         const RcView<double, true> gz{g.rc1 + base + j0 - 1, cs};
-#pragma unroll kReconUnroll
-        for (int v = 0; v < 7; v++) {
-          double al, ar;
-          recon_zone<double>(P.interp_order, win[sm][v][tid], win[s0][v][tid], win[sp][v][tid], gz, al, ar);
-          arb[v][tid] = ar;
-        }
+        recon_vars<7>(P.interp_order, gz, [&](int v, int q) { return win[q == 0 ? sm : q == 1 ? s0 : sp][v][tid]; },
+                      [&](int v, double, double hi) { arb[v][tid] = hi; });
       }
     }
 #pragma unroll 1
@@ -760,14 +741,8 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *_
         }
       } else {
         const RcView<double, true> gz{g.rc1 + base + j, cs};
-#pragma unroll kReconUnroll
-        for (int v = 0; v < 7; v++) {
-          pl[v] = arb[v][tid];
-          double al, ar;
-          recon_zone<double>(P.interp_order, win[sm][v][tid], win[s0][v][tid], win[sp][v][tid], gz, al, ar);
-          pr[v] = al;
-          arb[v][tid] = ar;
-        }
+        recon_vars<7>(P.interp_order, gz, [&](int v, int q) { return win[q == 0 ? sm : q == 1 ? s0 : sp][v][tid]; },
+                      [&](int v, double lo, double hi) { pl[v] = arb[v][tid]; pr[v] = lo; arb[v][tid] = hi; });
       }
       // zone k of row j that owns the sub-face, and the transverse_shock test of zone k
       const int dkj = dks(g, i, j), dkjm = dks(g, i, j - 1);
@@ -819,7 +794,7 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face1_kernel(const ProbDev *_
 // threads per warp instruction (0.36 ms a stage, plain FP64).
 constexpr int T2 = NT3 - 2;
 template <int STAGE, bool MIX>
-__global__ void __launch_bounds__(NT3, MDG_F3MINB) face2_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face2_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Seg2 *__restrict__ segs, int nseg,
                                                      const int *__restrict__ first, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
@@ -873,13 +848,8 @@ __global__ void __launch_bounds__(NT3, MDG_F3MINB) face2_kernel(const ProbDev *_
       }
     } else {
       const RcView<double, true> gz{g.rc2 + base + k0 - 1 + t, g.cols2};
-#pragma unroll kReconUnroll
-      for (int v = 0; v < 7; v++) {
-        double al, ar;
-        recon_zone<double>(P.interp_order, sv[v][t], sv[v][t + 1], sv[v][t + 2], gz, al, ar);
-        sal[v][t] = al;
-        sar[v][t] = ar;
-      }
+      recon_vars<7>(P.interp_order, gz, [&](int v, int q) { return sv[v][t + q]; },
+                    [&](int v, double lo, double hi) { sal[v][t] = lo; sar[v][t] = hi; });
     }
   }
   __syncthreads();
@@ -1124,9 +1094,11 @@ __global__ void __launch_bounds__(NT3, MDG_P3MINB) push3_kernel(const ProbDev *_
     }
     const double vol = geo3(g, G3_VOL, ij);
     const double pfact = STAGE ? 0.5 : 1.0, phfact = STAGE ? 0.5 : 0.0, ffact = STAGE ? 0.5 : 1.0;
+    double dv[NPRIM];
+    quotients<NPRIM>(divF, vol, dv);
 #pragma unroll
     for (int v = 0; v < NPRIM; v++) {
-      const double ddt = divF[v] / vol - src[v];
+      const double ddt = dv[v] - src[v];
       u[v] = pfact * u[v] + phfact * uh[v] - ffact * dt * ddt;
     }
     u_to_p(u, pf, geo3(g, G3_GCON + 0, ij), geo3(g, G3_GCON + 1, ij), geo3(g, G3_GCON + 2, ij), P.floors != 0,
@@ -1329,16 +1301,18 @@ static void build_runs(const Sweep3 &w, int dir, int run_len, RunList &out)
 {
   std::vector<Run3> runs;
   std::vector<int> cnt;
-  cut_runs(w, dir, fitting_run(w, run_len), runs, cnt);
+  run_len = fitting_run(w, run_len);
+  cut_runs(w, dir, run_len, runs, cnt);
   // long runs first (the tail of the launch is made of short ones), neighbouring rows in
   // neighbouring lanes: direction 0 by first face then theta row, direction 1 likewise
-  std::vector<int> ord(runs.size());
-  for (size_t q = 0; q < ord.size(); q++) ord[q] = (int)q;
-  std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
-    if (runs[a].nr != runs[b].nr) return runs[a].nr > runs[b].nr;
-    if (runs[a].r0 != runs[b].r0) return runs[a].r0 < runs[b].r0;
-    return runs[a].row < runs[b].row;
-  });
+  // (a counting sort on length and first face: the runs of a pair already come in row order)
+  int rmax = 0;
+  for (const Run3 &r : runs) rmax = std::max(rmax, r.r0);
+  auto bucket = [&](const Run3 &r) { return (size_t)(run_len - r.nr) * (rmax + 1) + r.r0; };
+  std::vector<int> pos((size_t)run_len * (rmax + 1) + 1, 0), ord(runs.size());
+  for (const Run3 &r : runs) pos[bucket(r) + 1]++;
+  for (size_t q = 1; q < pos.size(); q++) pos[q] += pos[q - 1];
+  for (size_t q = 0; q < runs.size(); q++) ord[pos[bucket(runs[q])]++] = (int)q;
   for (int q : ord) {
     Run3 r = runs[q];
     r.l0 = out.nlane;

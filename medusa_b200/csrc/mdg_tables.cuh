@@ -25,11 +25,14 @@ MDG_HD inline void rc_fields(double am, double a0, double ap, double bm, double 
   v[RC_GM] = gm; v[RC_G0] = g0; v[RC_GP] = gp;
   v[RC_XL] = xl; v[RC_XR] = xr;
   v[RC_DEN1] = den1; v[RC_DEN2] = den2;
-  v[RC_XLR] = xl - xr;
-  v[RC_XL2] = xl * xl; v[RC_XR2] = xr * xr;
-  v[RC_XMID] = 0.5 * (xl + xr);
   v[RC_DMR] = a0 + xr * (g0 * xr - 2.0 * b0);
   v[RC_DML] = a0 + xl * (g0 * xl - 2.0 * b0);
+  v[RC_RG0] = 1.0 / g0; v[RC_RDMR] = 1.0 / v[RC_DMR]; v[RC_RDML] = 1.0 / v[RC_DML];
+  const double xa = xl < 0.0 ? -xl : xl, xb = xr < 0.0 ? -xr : xr, big = 0x1p300, small = 0x1p-300;
+  auto fine = [&](double d) { const double m = d < 0.0 ? -d : d; return m > small && m < big; };
+  v[RC_XEPS] = (fine(g0) && fine(v[RC_DMR]) && fine(v[RC_DML]) && fine(xa > xb ? xa : xb))
+                   ? 0x1p-51 * (xa > xb ? xa : xb)
+                   : 1.0 / 0.0;
   v[RC_LSM] = xc - 0.5 * (xl + xm);
   v[RC_LSP] = 0.5 * (xr + xp) - xc;
   v[RC_LSC] = xp - xm;
