@@ -5,8 +5,9 @@
 Produces medusa_b200/_lib/libmedusa_b200.so (exports exactly the mdg_* entry points of
 include/medusa_b200.h).  The FP64 sweep translation units are compiled with
 -fmad=false and the host code with -ffp-contract=off: no multiply-add contraction, so
-every product and sum rounds as in the reference's CPU build.  The mixed-precision
-sweep (mdg_sweep1d_mixed.cu) is compiled with -use_fast_math instead.
+every product and sum rounds as in the reference's CPU build.  The mixed-precision sweeps
+have translation units of their own: the 1-D one with -use_fast_math, the 2-D and dendritic
+ones with -fmad=true.
 """
 from __future__ import annotations
 
@@ -25,16 +26,19 @@ LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libmedusa_b200.so")
 INCLUDE = os.path.join(ROOT, "include")
 
-SOURCES = ["mdg_capi.cu", "mdg_sweep1d.cu", "mdg_sweep1d_mixed.cu", "mdg_sweep2d.cu", "mdg_misc.cu",
-           "mdg_geometry.cpp", "mdg_noalloc.cu", "mdg_server.cu", "mdg_tables.cu", "mdg_sweep3d.cu", "mdg_tma.cu",
-           "mdg_eos_table.cu"]
+SOURCES = ["mdg_capi.cu", "mdg_sweep1d.cu", "mdg_sweep1d_mixed.cu", "mdg_sweep2d.cu", "mdg_sweep2d_mixed.cu",
+           "mdg_misc.cu", "mdg_geometry.cpp", "mdg_noalloc.cu", "mdg_server.cu", "mdg_tables.cu", "mdg_sweep3d.cu",
+           "mdg_sweep3d_mixed.cu", "mdg_tma.cu", "mdg_eos_table.cu"]
 HEADERS = ["mdg_internal.h", "mdg_recon.h", "mdg_hydro.cuh", "mdg_kernels.cuh", "mdg_load1d.cuh", "mdg_tables.cuh",
-           "mdg_grid3d.cuh", "mdg_mixed.cuh", "mdg_tma.cuh",
+           "mdg_grid3d.cuh", "mdg_mixed.cuh", "mdg_sweep2d.cuh", "mdg_sweep3d.cuh", "mdg_tma.cuh",
            "mdg_timeloop.cuh"]
 # The mixed-precision sweep: fast FP32 division/square root and multiply-add contraction
 # (its FP64 parts are not required to round like the reference's).
-MIXED_FLAGS = ["-use_fast_math"]
-FLAGS = {"mdg_sweep1d_mixed.cu": MIXED_FLAGS}
+MIXED_FLAGS = ["-use_fast_math", "-DMDG_FAST_MATH32"]
+# The mixed 2-D and dendritic sweeps: multiply-add contraction, functions at full accuracy.
+MIXED2_FLAGS = ["-fmad=true"]
+FLAGS = {"mdg_sweep1d_mixed.cu": MIXED_FLAGS, "mdg_sweep2d_mixed.cu": MIXED2_FLAGS,
+         "mdg_sweep3d_mixed.cu": MIXED2_FLAGS}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -116,15 +116,51 @@ __device__ __forceinline__ GamConst<T> gam_const(T G)
   return c;
 }
 
+// Quotient and square root of the wave-speed estimate.  FP64: the operators (correctly rounded).
+// FP32: the approximate reciprocal (reciprocal square root) and one correction by the exact
+// remainder, a Newton step: within half an ulp and a little, as the rounded operators for the
+// purposes of an FP32 estimate, without their range checks and calls (a zero or infinite
+// divisor gives NaN, where the operator gives an infinity or zero).  The 1-D mixed sweep's
+// fast-math translation unit keeps its approximate operators.
+__device__ __forceinline__ double quot(double a, double b) { return a / b; }
+__device__ __forceinline__ double root(double x) { return sqrt(x); }
+__device__ __forceinline__ float quot(float a, float b)
+{
+#ifdef MDG_FAST_MATH32
+  return a / b;
+#else
+  float y;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(b));
+  const float q = a * y;
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+#endif
+}
+__device__ __forceinline__ float root(float x)
+{
+#ifdef MDG_FAST_MATH32
+  return sqrtf(x);
+#else
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  const float g = x * y;
+  return (x == 0.0f) ? x : __fmaf_rn(__fmaf_rn(-g, g, x), 0.5f * y, g);
+#endif
+}
+
 // The two tests that the solvers make on a face's pressure ratio: (p_max - p_min) / p_min >
 // 0.5 (shock tag) and p_max / p_min < 2.  In FP64, for positive p_min, fl(x / y) > 0.5 exactly
 // when x > 0.5 y and fl(x / y) < 2 exactly when x < 2 y: the quotient of two numbers that
 // differ from the ratio 1/2 or 2 at all differs by more than the half ulp that rounding
-// could close.  (FP32 keeps its approximate quotients.)
+// could close.  (The fast-math FP32 sweep keeps its approximate quotients.)
 template <typename T>
 __device__ __forceinline__ void pressure_ratio_tests(T p_max, T p_min, bool &below2, int &isshock)
 {
-  if (sizeof(T) == 8 && p_min > T(0x1p-100) * T(0x1p-100) && p_max < T(0x1p120) * T(0x1p120)) {
+#ifdef MDG_FAST_MATH32
+  constexpr bool compare = sizeof(T) == 8;
+#else
+  constexpr bool compare = true;
+#endif
+  if (compare && p_min > T(0x1p-100) && p_max < T(0x1p120)) {
     below2 = p_max < T(2) * p_min;
     isshock = (p_max - p_min > T(0.5) * p_min) ? 1 : 0;
   } else {
@@ -133,12 +169,12 @@ __device__ __forceinline__ void pressure_ratio_tests(T p_max, T p_min, bool &bel
   }
 }
 
-// q[v] = a[v] / b, correctly rounded, by one reciprocal (div_by): a zero numerator is its
+// q[v] = a[v] / b (q not a), correctly rounded, by one reciprocal (div_by): a zero numerator is its
 // own quotient for b > 0; numbers outside recon_in_range and b <= 0 take the division.
 // MIX (the mixed sweeps, whose results are not pinned to the reference's rounding): the
 // product with the reciprocal.
 template <int N>
-__device__ __noinline__ void quotients_declined(const double (&a)[N], double b, double (&q)[N])
+__device__ __noinline__ void quotients_declined(const double *a, double b, double *q)
 {
   for (int v = 0; v < N; v++) q[v] = a[v] / b;
 }
@@ -161,6 +197,20 @@ __device__ __forceinline__ void quotients(const double (&a)[N], double b, double
   if (!ok) quotients_declined<N>(a, b, q);
 }
 
+// x^y of the two-rarefaction estimate.  FP32 (the mixed sweeps): exp(y log x) where its
+// exponent is small, |y log x| <= 1/2, so that the rounding of the product adds at most half an
+// ulp to the 1-2 ulps of the two functions (powf: up to 4 ulps); powf elsewhere.
+__device__ __forceinline__ double pow_rarefaction(double x, double y) { return pow(x, y); }
+__device__ __forceinline__ float pow_rarefaction(float x, float y)
+{
+#ifdef MDG_FAST_MATH32
+  return powf(x, y);   // (the 1-D mixed sweep's approximate form)
+#else
+  const float z = y * logf(x);
+  return (fabsf(z) <= 0.5f) ? expf(z) : powf(x, y);
+#endif
+}
+
 // Wave-speed estimate shared by HLLC and HLLE (riemann.c:368-429 / 210-303).
 // w[0..4] primitives, w[5] pressure (w[6], Gamma, equals gc.g).
 template <typename T>
@@ -168,8 +218,8 @@ __device__ __forceinline__ void wave_speeds(const T *pl, const T *pr, T u_l, T u
                                             const GamConst<T> &gc, T &sl, T &sr, T &ss, T &p_s, int &isshock)
 {
   const T p_l = pl[5], p_r = pr[5], G = gc.g;
-  T cs_l = sqrt(G * p_l / pl[RHO]);
-  T cs_r = sqrt(G * p_r / pr[RHO]);
+  T cs_l = root(quot(G * p_l, pl[RHO]));
+  T cs_r = root(quot(G * p_r, pr[RHO]));
   T p_max, p_min;
   if (p_l > p_r) { p_max = p_l; p_min = p_r; } else { p_max = p_r; p_min = p_l; }
   bool below2;
@@ -182,30 +232,30 @@ __device__ __forceinline__ void wave_speeds(const T *pl, const T *pr, T u_l, T u
     // primitive-variable estimate kept
   } else if (p_s < p_min) {
     // two rarefactions (Toro 9.35-9.36)
-    T plr = pow(p_l / p_r, gc.ce);
-    T s0 = (plr * u_l / cs_l + u_r / cs_r + T(2) * (plr - T(1)) / gc.gm1) / (plr / cs_l + T(1) / cs_r);
-    p_s = T(0.5) * (p_l * pow(T(1) + gc.gm1 / (T(2) * cs_l) * (u_l - s0), gc.cx)
-                  + p_r * pow(T(1) + gc.gm1 / (T(2) * cs_r) * (s0 - u_r), gc.cx));
+    T plr = pow_rarefaction(quot(p_l, p_r), gc.ce);
+    T s0 = quot(quot(plr * u_l, cs_l) + quot(u_r, cs_r) + quot(T(2) * (plr - T(1)), gc.gm1), quot(plr, cs_l) + quot(T(1), cs_r));
+    p_s = T(0.5) * (p_l * pow_rarefaction(T(1) + quot(gc.gm1, T(2) * cs_l) * (u_l - s0), gc.cx)
+                  + p_r * pow_rarefaction(T(1) + quot(gc.gm1, T(2) * cs_r) * (s0 - u_r), gc.cx));
     p_s = tmax(p_s, T(0));
   } else {
     // two shocks (Toro 9.42-9.43)
-    T a_l = T(2) / (gc.gp1 * pl[RHO]);
-    T a_r = T(2) / (gc.gp1 * pr[RHO]);
+    T a_l = quot(T(2), gc.gp1 * pl[RHO]);
+    T a_r = quot(T(2), gc.gp1 * pr[RHO]);
     T b_l = gc.cb * p_l;
     T b_r = gc.cb * p_r;
-    T g_l = sqrt(a_l / (p_s + b_l));
-    T g_r = sqrt(a_r / (p_s + b_r));
-    p_s = (g_l * p_l + g_r * p_r - (u_r - u_l)) / (g_l + g_r);
+    T g_l = root(quot(a_l, p_s + b_l));
+    T g_r = root(quot(a_r, p_s + b_r));
+    p_s = quot(g_l * p_l + g_r * p_r - (u_r - u_l), g_l + g_r);
     p_s = tmax(p_s, T(0));
   }
   // q = 1 when p_s <= p, else sqrt(1 + (G+1)/(2G) (p_s/p - 1)); sqrt(1) == 1 exactly, so
   // the square root is taken unconditionally on the selected argument (no branch)
-  T q_l = sqrt((p_s <= p_l) ? T(1) : T(1) + gc.cq * (p_s / p_l - T(1)));
-  T q_r = sqrt((p_s <= p_r) ? T(1) : T(1) + gc.cq * (p_s / p_r - T(1)));
+  T q_l = root((p_s <= p_l) ? T(1) : T(1) + gc.cq * (quot(p_s, p_l) - T(1)));
+  T q_r = root((p_s <= p_r) ? T(1) : T(1) + gc.cq * (quot(p_s, p_r) - T(1)));
   sl = u_l - cs_l * q_l;
   sr = u_r + cs_r * q_r;
-  ss = (p_r - p_l + pl[RHO] * u_l * (sl - u_l) - pr[RHO] * u_r * (sr - u_r))
-     / (pl[RHO] * (sl - u_l) - pr[RHO] * (sr - u_r));
+  ss = quot(p_r - p_l + pl[RHO] * u_l * (sl - u_l) - pr[RHO] * u_r * (sr - u_r),
+            pl[RHO] * (sl - u_l) - pr[RHO] * (sr - u_r));
 }
 
 // p_uflux (riemann.c:4-37) for direction DIR

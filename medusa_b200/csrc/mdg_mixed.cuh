@@ -45,7 +45,7 @@ __device__ __forceinline__ void mixed_recon(float dqm, float dqp, const MixW &w,
   // re-fit and move an interior extremum to the nearer edge (reconstruct.c:174-200)
   const float A2 = w.eal * l + w.ear * r;
   const float B2 = w.ebl * l + w.ebr * r;
-  const float s = -B2 / (2.0f * A2);
+  const float s = quot(-B2, 2.0f * A2);
   if (s > 0.0f && s < w.dxz) {
     if (s > 0.5f * w.dxz) l = r * w.mr;
     else r = l * w.ml;
@@ -91,7 +91,7 @@ __device__ __forceinline__ bool riemann_hllc_mixed(const double *pl, const doubl
   wave_speeds<float>(plf, prf, u_l, u_r, false, gc, sl, sr, ss, p_s, isshock);
   if (ss > sr) sr = 1.001f * ss;
   if (ss < sl) sl = 1.001f * ss;
-  sig = fmaxf(fabsf(sl), fabsf(sr)) / sc;
+  sig = quot(fmaxf(fabsf(sl), fabsf(sr)), sc);
   if (sl > 0.0f) { pflux<DIR, false, double>(pl, pl[5], g, flux); return true; }
   if (sr < 0.0f) { pflux<DIR, false, double>(pr, pr[5], g, flux); return true; }
   const float emax = fmaxf(plf[RHO] * u_l * u_l + plf[5], prf[RHO] * u_r * u_r + prf[5]);
@@ -107,7 +107,7 @@ __device__ __forceinline__ bool riemann_hllc_mixed(const double *pl, const doubl
   //   rho* - rho = rho (ss-uk)/(sk-ss),  E* - E = (E (ss-uk) + p* ss - p uk)/(sk-ss)
   const float rk = left ? plf[RHO] : prf[RHO];
   const float pkf = left ? plf[5] : prf[5];
-  const float inv = 1.0f / (sk - ss);
+  const float inv = quot(1.0f, sk - ss);
   const float dU0 = rk * (ss - uk) * inv;
   const float dUE = ((float)u[UU] * (ss - uk) + p_s * ss - pkf * uk) * inv;
   double dU[NPRIM];
@@ -116,8 +116,8 @@ __device__ __forceinline__ bool riemann_hllc_mixed(const double *pl, const doubl
   const double gd[3] = {g.g0, g.g1, g.g2};
 #pragma unroll
   for (int m = 0; m < 3; m++)   // normal component: (ss-uk) rho + ss (rho*-rho), over the scale
-    dU[U1 + m] = (m == DIR) ? gd[m] * (double)(((ss - uk) * rk + ss * dU0) / sc) : gd[m] * pk[U1 + m] * (double)dU0;
-  const double slr = (double)(sk / sc);
+    dU[U1 + m] = (m == DIR) ? gd[m] * (double)quot((ss - uk) * rk + ss * dU0, sc) : gd[m] * pk[U1 + m] * (double)dU0;
+  const double slr = (double)quot(sk, sc);
 #pragma unroll
   for (int v = 0; v < NPRIM; v++) flux[v] = g.area * (fx[v] + slr * dU[v]);
   return true;
