@@ -341,7 +341,13 @@ void mdg::make_probdev(const mdg_problem_desc &d, ProbDev &P)
   P.grav_on = (d.grav[0] != 0.0 || d.grav[1] != 0.0 || d.grav[2] != 0.0);
   P.x0 = d.startx[0];
   P.mono = d.monopole;
-  if (d.ndim == 1 && d.geom == MDG_SPHERICAL) spherical_1d_constants(P.gk_area, P.gk_th1, P.gk_th2, P.gk_tc);
+  if (d.ndim == 1 && d.geom == MDG_SPHERICAL) {
+    spherical_1d_constants(P.gk_area, P.gk_th1, P.gk_th2, P.gk_tc);
+    P.gk_iarea = 1.0 / P.gk_area;
+    P.gk_ith1 = 1.0 / P.gk_th1;
+    P.gk_ith2 = 1.0 / P.gk_th2;
+  }
+  P.idx0 = 1.0 / P.dx0;
   if (d.ndim == 1 && d.prob_kind == MDG_PROB_DUST) dust_ghost_u1(d, P.u1_hi);
 }
 

@@ -491,19 +491,28 @@ __device__ __forceinline__ double eos_press(int eos, double gam, double Kpoly, d
   return (eos == 0) ? (gam - 1.0) * uu : Kpoly * pow(rho, gam);
 }
 
-// Block-wide min of a double, folded into an order-preserving atomic accumulator.
+// Smallest of a full warp's keys: the integer reduction unit on the high and then the low words
+// (4 instructions for the 25 of a shuffle tree of doubles).
+__device__ __forceinline__ unsigned long long warp_min_ord(unsigned long long k)
+{
+  const unsigned h = (unsigned)(k >> 32), hm = __reduce_min_sync(0xffffffffu, h);
+  const unsigned lm = __reduce_min_sync(0xffffffffu, h == hm ? (unsigned)k : 0xffffffffu);
+  return ((unsigned long long)hm << 32) | lm;
+}
+
+// Block-wide min of a double, folded into an order-preserving atomic accumulator (a NaN counts
+// as 1e300: the state it comes from is flagged by flag_nonfinite).  sbuf: one double per warp.
 __device__ __forceinline__ void block_min_to(double v, unsigned long long *acc, double *sbuf)
 {
-  for (int o = 16; o > 0; o >>= 1) v = tmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+  unsigned long long *sk = reinterpret_cast<unsigned long long *>(sbuf);
+  unsigned long long k = warp_min_ord(dbl_to_ord(v == v ? v : 1.0e300));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sbuf[warp] = v;
+  if (lane == 0) sk[warp] = k;
   __syncthreads();
   if (warp == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    v = (lane < nw) ? sbuf[lane] : 1.0e300;
-    for (int o = 16; o > 0; o >>= 1) v = tmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) atomicMin(acc, dbl_to_ord(v));
+    k = warp_min_ord(lane < nw ? sk[lane] : ~0ull);
+    if (lane == 0) atomicMin(acc, k);
   }
 }
 

@@ -104,6 +104,7 @@ struct ProbDev {
   // 1-D geometry in closed form (mixed-precision sweep): lower edge of zone 0 and the
   // angular integrals of the 1-D spherical metric (spherical_1d_constants)
   double x0, gk_area, gk_th1, gk_th2, gk_tc;
+  double gk_iarea, gk_ith1, gk_ith2, idx0;   // reciprocals of gk_area, gk_th1, gk_th2, dx0
 };
 
 // Time bookkeeping of one problem, resident on the device.
