@@ -57,6 +57,22 @@ __device__ __noinline__ FacePair recon_declined(double am, double a, double ap, 
   return o;
 }
 
+// One variable of one zone in order `order`.
+template <typename G>
+__device__ __forceinline__ FacePair recon_var(int order, double am, double a, double ap, const G &g)
+{
+  FacePair o;
+  if (order == 3) {
+    if (!para_recon_fast(am, a, ap, g, o.al, o.ar)) o = recon_declined<G>(am, a, ap, g);
+  } else if (order == 2) {
+    lin_recon_zone(am, a, ap, g, o.al, o.ar);
+  } else {
+    o.al = a;
+    o.ar = a;
+  }
+  return o;
+}
+
 // NV variables of one zone in order `order`: at(v, q) is variable v's average in zone i-1+q,
 // put(v, al, ar) takes its face values.  The loop is not unrolled: one copy of the code per
 // loop keeps the kernels in the instruction cache.
@@ -65,16 +81,7 @@ __device__ __forceinline__ void recon_vars(int order, const G &g, At at, Put put
 {
 #pragma unroll 1
   for (int v = 0; v < NV; v++) {
-    const double am = at(v, 0), a = at(v, 1), ap = at(v, 2);
-    FacePair o;
-    if (order == 3) {
-      if (!para_recon_fast(am, a, ap, g, o.al, o.ar)) o = recon_declined<G>(am, a, ap, g);
-    } else if (order == 2) {
-      lin_recon_zone(am, a, ap, g, o.al, o.ar);
-    } else {
-      o.al = a;
-      o.ar = a;
-    }
+    const FacePair o = recon_var(order, at(v, 0), at(v, 1), at(v, 2), g);
     put(v, o.al, o.ar);
   }
 }
@@ -502,6 +509,8 @@ __device__ __forceinline__ unsigned long long warp_min_ord(unsigned long long k)
 
 // Block-wide min of a double, folded into an order-preserving atomic accumulator (a NaN counts
 // as 1e300: the state it comes from is flagged by flag_nonfinite).  sbuf: one double per warp.
+// OWN: the accumulator is the block's alone (shared memory), so a plain minimum will do.
+template <bool OWN = false>
 __device__ __forceinline__ void block_min_to(double v, unsigned long long *acc, double *sbuf)
 {
   unsigned long long *sk = reinterpret_cast<unsigned long long *>(sbuf);
@@ -512,7 +521,10 @@ __device__ __forceinline__ void block_min_to(double v, unsigned long long *acc, 
   if (warp == 0) {
     const int nw = (blockDim.x + 31) >> 5;
     k = warp_min_ord(lane < nw ? sk[lane] : ~0ull);
-    if (lane == 0) atomicMin(acc, k);
+    if (lane == 0) {
+      if (OWN) *acc = k < *acc ? k : *acc;
+      else atomicMin(acc, k);
+    }
   }
 }
 

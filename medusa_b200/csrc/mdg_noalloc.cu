@@ -200,7 +200,15 @@ extern "C" int mdg_advance_1d_noalloc(const mdg_problem_desc *desc, const double
 
   launch_reset_time(times, 0, st);
   launch_initial_estimate_one(probs, times, 0, n1, tb, S, st);
-  for (int k = 0; k < nsteps; k++) {
+  // the resident stepper where the problem fits a thread-block cluster, else four launches a
+  // step (the same bits): 20 steps of 200 zones 0.88 -> 0.75 ms a call
+  bool wide = false;
+  const int cs = resident1d_cluster_size(ntiles, 1, &wide);
+  for (int k = 0; k < nsteps && cs > 0; k += RESIDENT_STEPS) {
+    const int n = nsteps - k < RESIDENT_STEPS ? nsteps - k : RESIDENT_STEPS;
+    CKN(launch_resident1d(cs, wide, 1, probs, times, tb, S, PH, n, err, st));
+  }
+  for (int k = 0; k < nsteps && cs == 0; k++) {
     launch_dt_finalize(probs, times, 1, err, st);
     launch_stage1d(0, probs, times, tiles, ntiles, tb, S, S, PH, st);
     launch_stage1d(1, probs, times, tiles, ntiles, tb, PH, S, S, st);

@@ -31,13 +31,18 @@ namespace mdg {
 // (GF_TMA_ROWS rows) arrive in shared memory by two tensor loads issued at the start,
 // which overlap the state loads; otherwise every field is read from the tables in HBM
 // when used.  The results are the same.
-// One RK stage of one tile (run by the NT1 threads of a CTA).  tm: the tensor maps of
-// the tables (a __grid_constant__ kernel parameter; not read without TMA).
-template <int STAGE, bool TMA>
-__device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
-                                             const Tile tile, const Tables &tb, const StateSoA &sst,
-                                             const StateSoA &sn, const StateSoA &out, const TmaTables1d &tm)
+// One RK stage of one tile, run by the NT1 x G threads of a CTA: thread t of group 0 does zone
+// t of the tile; with G = 4 the groups share the six variables' reconstructions of every zone
+// (density / internal energy / v1 and v2 / pressure and v3).  dt, t_bc: the step and the time the
+// boundaries see; minacc: the CFL accumulator (OWN: this CTA's alone); T: the problem's record (error mark).  tm: the
+// tensor maps of the tables (a __grid_constant__ kernel parameter; not read without TMA).
+template <int STAGE, bool TMA, int G, bool OWN>
+__device__ __forceinline__ void stage1d_tile(const ProbDev &P, ProbTime *T, double dt, double t_bc,
+                                             unsigned long long *minacc, const Tile tile, const Tables &tb,
+                                             const StateSoA &sst, const StateSoA &sn, const StateSoA &out,
+                                             const TmaTables1d &tm)
 {
+  static_assert(G == 1 || (G == 4 && !TMA), "one thread per zone, or four without TMA");
   __shared__ double sv[6][NT1 + 2];     // stage-state pencil: 5 primitives + pressure
   __shared__ double sred[32];
   __shared__ __align__(128) double s_rc[TMA ? RC_TMA_ROWS : 1][TMA ? TMA_COLS1 : 1];
@@ -51,11 +56,8 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
   double (*sar)[NT1] = TMA ? reinterpret_cast<double(*)[NT1]>(&s_rc[0][0]) : sar_own;
   double (*sfl)[NT1] = TMA ? reinterpret_cast<double(*)[NT1]>(&s_rc[0][0] + 6 * NT1) : sfl_own;
 
-  if (times[tile.prob].done) return;   // past tmax: the time loop has ended (CTA-uniform)
-  const ProbDev &P = probs[tile.prob];
-  const double dt = times[tile.prob].dt;
-  const double t_bc = STAGE ? times[tile.prob].t_bc1 : times[tile.prob].t;
-  const int t = threadIdx.x;
+  __shared__ double sal[G > 1 ? 6 : 1][G > 1 ? NT1 : 1];   // left face values (G > 1: other groups' threads)
+  const int t = G > 1 ? threadIdx.x % NT1 : threadIdx.x, grp = G > 1 ? threadIdx.x / NT1 : 0;
   const int n1 = P.n1;
   const int z = tile.i0 - 1 + t;           // zone reconstructed by this thread
   const double *rc = tb.rc0;
@@ -80,17 +82,20 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     return __ldg(geo + f * gs + c);
   };
 
-  double w[6];
-  load_cell_1d(P, sst, rc, rcs, z, t_bc, w);
+  if (grp == 0) {
+    double w[6];
+    load_cell_1d(P, sst, rc, rcs, z, t_bc, w);
 #pragma unroll
-  for (int v = 0; v < 6; v++) sv[v][t + 1] = w[v];
-  if (t == 0) {
+    for (int v = 0; v < 6; v++) sv[v][t + 1] = w[v];
+  }
+  // the outer columns (with several groups, by threads that load nothing else)
+  if (t == 0 && grp == G - 1) {
     double w2[6];
     load_cell_1d(P, sst, rc, rcs, tile.i0 - 2, t_bc, w2);
 #pragma unroll
     for (int v = 0; v < 6; v++) sv[v][0] = w2[v];
   }
-  if (t == NT1 - 1) {
+  if (t == NT1 - 1 && grp == G - 1) {
     double w2[6];
     load_cell_1d(P, sst, rc, rcs, tile.i0 + NT1 - 1, t_bc, w2);
 #pragma unroll
@@ -101,7 +106,7 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     // problem and the CTA leaves after waiting once more, as bounded)
     const bool ok = mbar_wait(&s_bar, 0);
     if (__syncthreads_or(!ok)) {
-      if (t == 0) times[tile.prob].err = MDG_ERR_INTERNAL;
+      if (t == 0) T->err = MDG_ERR_INTERNAL;
       mbar_wait(&s_bar, 0);
       return;
     }
@@ -111,7 +116,17 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
   // reconstruct zone z once (interp(), reconstruct.c:225-279); Gamma is the constant
   // adiabatic index, which every order reconstructs to itself.
   double al[7], ar[7];
-  {
+  if (G > 1) {
+    const int zc = z < -1 ? -1 : (z > n1 ? n1 : z);
+    const RcView<double, true> g{rc + P.geo_off + zc + NG, rcs};
+    const int first = grp == 3 ? 5 : grp, second = grp < 2 ? -1 : grp + 1;
+#pragma unroll 1
+    for (int v = first; v >= 0; v = (v == first) ? second : -1) {
+      const FacePair o = recon_var(P.interp_order, sv[v][t], sv[v][t + 1], sv[v][t + 2], g);
+      sal[v][t] = o.al;
+      sar[v][t] = o.ar;
+    }
+  } else {
     int zc = z < -1 ? -1 : (z > n1 ? n1 : z);
     const int64_t c = P.geo_off + zc + NG;
     const RcView<double, !TMA> g{TMA ? &s_rc[0][c - bx] : rc + c, TMA ? (int64_t)TMA_COLS1 : rcs};
@@ -120,16 +135,23 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     al[6] = P.gam; ar[6] = P.gam;
   }
   if (TMA) __syncthreads();   // every zone reconstructed: the recon rows may be overwritten
+  if (G == 1) {
 #pragma unroll
-  for (int v = 0; v < 6; v++) sar[v][t] = ar[v];
+    for (int v = 0; v < 6; v++) sar[v][t] = ar[v];
+  }
   __syncthreads();
+  if (G > 1 && grp == 0) {
+#pragma unroll
+    for (int v = 0; v < 6; v++) al[v] = sal[v][t];
+    al[6] = P.gam;
+  }
 
   double lmin = 1.0e300;
   double smax = 0.0, nmin = 1.0e300, lmax = 0.0;
   const GamConst<double> gc = gam_const(P.gam);
   // face z: between zones z-1 and z (pl = right state of z-1, pr = left state of z)
   const bool face_ok = (t >= 1) && (z >= 0) && (z <= n1);
-  if (t >= 1) {
+  if (t >= 1 && grp == 0) {
     double pl[7], flux[NPRIM], sig;
 #pragma unroll
     for (int v = 0; v < 6; v++) pl[v] = sar[v][t - 1];
@@ -150,7 +172,7 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
   __syncthreads();
 
   // push() for zone z (step.c:380-470)
-  if (t >= 1 && t <= NT1 - 2 && z >= 0 && z < n1) {
+  if (grp == 0 && t >= 1 && t <= NT1 - 2 && z >= 0 && z < n1) {
     const int64_t gi = P.geo_off + z + NG;
     const int64_t cell = P.cell_off + z;
     double ph[NPRIM], pn[NPRIM], u[NPRIM], uh[NPRIM], src[NPRIM], divF[NPRIM], pf[NPRIM];
@@ -200,7 +222,7 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
     u_to_p(u, pf, gf(GF_GC0, gi), gf(GF_GC1, gi), gf(GF_GC2, gi), P.floors != 0, P.rho_floor, P.e_floor);
 #pragma unroll
     for (int v = 0; v < NPRIM; v++) out.v[v][cell] = pf[v];
-    flag_nonfinite(pf, &times[tile.prob]);
+    flag_nonfinite(pf, T);
     if (STAGE == 1) {
       // zone term of the next estimate_dt (step.c:177-187): velocity of the new state,
       // sound speed of the stage state (sim_eos was last filled from sim_ph)
@@ -212,10 +234,12 @@ __device__ __forceinline__ void stage1d_tile(const ProbDev *__restrict__ probs, 
   }
   // min of dx/|sig| over faces, of the zero-source limits and of 1/local_dt, each taken
   // on its numerator or denominator (monotone division, see src_dt_numerator_min)
-  lmin = tmin(lmin, P.dx0 / smax);
-  lmin = tmin(lmin, src_dt_from_numerator(nmin));
-  if (STAGE == 1) lmin = tmin(lmin, 1.0 / lmax);
-  block_min_to(lmin, &times[tile.prob].minacc, sred);
+  if (grp == 0) {
+    lmin = tmin(lmin, P.dx0 / smax);
+    lmin = tmin(lmin, src_dt_from_numerator(nmin));
+    if (STAGE == 1) lmin = tmin(lmin, 1.0 / lmax);
+  }
+  block_min_to<OWN>(lmin, minacc, sred);
 }
 
 template <int STAGE, bool TMA>
@@ -224,50 +248,93 @@ stage1d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                const Tile *__restrict__ tiles, Tables tb, StateSoA sst, StateSoA sn, StateSoA out,
                const __grid_constant__ TmaTables1d tm)
 {
-  stage1d_tile<STAGE, TMA>(probs, times, tiles[blockIdx.x], tb, sst, sn, out, tm);
+  const Tile tile = tiles[blockIdx.x];
+  ProbTime *T = times + tile.prob;
+  if (T->done) return;   // past tmax: the time loop has ended (CTA-uniform)
+  stage1d_tile<STAGE, TMA, 1, false>(probs[tile.prob], T, T->dt, STAGE ? T->t_bc1 : T->t, &T->minacc, tile, tb, sst, sn, out,
+                              tm);
 }
 
 // The resident stepper: nsteps steps of every problem, cluster c advancing problem c with
 // CTA r on the tile of zones [126 r, 126 r + 126) (CTAs past the last zone only take part
-// in the barriers).  Each step: the dt rules (one thread), stage 0 (p -> ph), stage 1
-// (ph, p -> p), the time update (one thread); a cluster barrier after the dt rules and
-// after each stage orders the state, the time record and the CFL accumulator between the
-// CTAs (release/acquire at cluster scope).  Every CTA of a cluster takes the same
-// barriers: the loop runs nsteps iterations unless the problem's loop has ended (t >=
-// tmax), which every CTA reads from the time record after the same barrier -- the next
-// write of that flag comes two barriers later -- so all leave together; the lead then
-// closes the step as the time update would (a step past the end changes nothing else).
-__global__ void __launch_bounds__(NT1)
+// in the barriers).  Every CTA keeps the problem's time record in shared memory and runs the
+// time rules on its own copy (the same arithmetic on the same numbers, so the copies agree);
+// what the CTAs exchange is the state, through global memory, and their tiles' CFL minima, which
+// each CTA keeps in its shared memory, in two words that take turns, and reads from the others'
+// (distributed shared memory, plain loads).  Each step: the dt rules, stage 0 (p -> ph), a
+// cluster barrier, stage 1 (ph, p -> p), a cluster barrier, the time update (the barriers release
+// and acquire at cluster scope).  A step's word is read after its last barrier and cleared by
+// its owner after the next one, one barrier before its next use.  Every CTA
+// takes the same barriers: the loop runs nsteps iterations unless the problem's loop has ended
+// (t >= tmax), which every copy of the record says at the same step.  CTA 0 writes the record
+// back at the end.
+//
+// G threads per zone: a stage of so few zones is a chain of dependent FP64 operations, and the
+// six reconstructions were a third of it one after the other.  With a CTA per SM (G = 4, all
+// clusters resident at once) the groups run them side by side.  Together with the record
+// copies (two barriers a step for three, no thread that the others wait for): Sod 1024 23.5 ->
+// 21.1 us per step.
+template <int G>
+__global__ void __launch_bounds__(NT1 * G, G > 1 ? 1 : 3)
 resident1d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times, Tables tb, StateSoA p,
                   StateSoA ph, int nsteps, int *err, const __grid_constant__ TmaTables1d none)
 {
   namespace cg = cooperative_groups;
+  __shared__ ProbTime rec;
+  __shared__ unsigned long long acc[2];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int m = (int)(blockIdx.x / cl.num_blocks());
+  const ProbDev &P = probs[m];
   const Tile tile{m, rank * TILE1, 0, 0};
-  const bool active = tile.i0 < probs[m].n1;
-  const bool lead = rank == 0 && threadIdx.x == 0;
-  for (int k = 0; k < nsteps; k++) {
-    if (lead) dt_finalize_one(probs[m], times + m, err);
-    cl.sync();
-    if (times[m].done) {
-      if (lead) finish_one(times + m);
-      break;
-    }
-    if (active) stage1d_tile<0, false>(probs, times, tile, tb, p, p, ph, none);
-    cl.sync();
-    if (active) stage1d_tile<1, false>(probs, times, tile, tb, ph, p, p, none);
-    cl.sync();
-    if (lead) finish_one(times + m);
+  const bool active = tile.i0 < P.n1, first = threadIdx.x == 0;
+  const int lane = (int)threadIdx.x, ncta = (int)cl.num_blocks();
+  // the smallest of the CTAs' words w (run by warp 0)
+  auto cluster_min = [&](int w) {
+    const unsigned long long v = lane < ncta ? *cl.map_shared_rank(acc + w, lane < ncta ? lane : 0) : ~0ull;
+    return warp_min_ord(v);
+  };
+  if (first) {
+    rec = times[m];
+    acc[0] = acc[1] = dbl_to_ord(1.0e100);
   }
+  cl.sync();
+  int k = 0;
+  for (; k < nsteps; k++) {
+    unsigned long long *mine = acc + (k & 1), *last = acc + ((k + 1) & 1);
+    if (threadIdx.x < 32) {
+      const unsigned long long min_last = k > 0 ? cluster_min((k + 1) & 1) : 0ull;
+      if (first) {
+        if (k > 0) rec.minacc = min_last;
+        dt_finalize_one(P, &rec, err);
+      }
+    }
+    __syncthreads();
+    if (rec.done) break;
+    if (active) stage1d_tile<0, false, G, true>(P, times + m, rec.dt, rec.t, mine, tile, tb, p, p, ph, none);
+    cl.sync();
+    if (first) *last = dbl_to_ord(1.0e100);                // every CTA has read it
+    if (active) stage1d_tile<1, false, G, true>(P, times + m, rec.dt, rec.t_bc1, mine, tile, tb, ph, p, p, none);
+    cl.sync();
+    if (first) finish_one(&rec);
+  }
+  const unsigned long long min_end = threadIdx.x < 32 ? cluster_min((k + 1) & 1) : 0ull;
+  if (first && rank == 0) {
+    if (k < nsteps) finish_one(&rec);                      // the loop has ended: as a step past it
+    else rec.minacc = min_end;
+    ProbTime *T = times + m;
+    T->t = rec.t; T->dt = rec.dt; T->dtold = rec.dtold; T->t_bc1 = rec.t_bc1; T->t_next = rec.t_next;
+    T->minacc = rec.minacc; T->istep = rec.istep; T->dt_ready = rec.dt_ready; T->done = rec.done;
+    if (rec.err) T->err = rec.err;                         // (the tiles mark non-finite states in *T)
+  }
+  cl.sync();                                               // the CTAs' words outlive every reader
 }
 
-static cudaLaunchConfig_t resident1d_config(int cs, int nprob, cudaStream_t st, cudaLaunchAttribute *attr)
+static cudaLaunchConfig_t resident1d_config(int cs, int nprob, bool wide, cudaStream_t st, cudaLaunchAttribute *attr)
 {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)(cs * nprob), 1, 1);
-  c.blockDim = dim3(NT1, 1, 1);
+  c.blockDim = dim3(wide ? 4 * NT1 : NT1, 1, 1);
   c.dynamicSmemBytes = 0;
   c.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -279,34 +346,45 @@ static cudaLaunchConfig_t resident1d_config(int cs, int nprob, cudaStream_t st, 
   return c;
 }
 
-int resident1d_cluster_size(int max_tiles)
+// Clusters of cs CTAs that the device holds at once (0: none, or the query failed).
+static int resident1d_clusters(int cs, bool wide)
 {
-  if (max_tiles < 1 || max_tiles > RESIDENT1D_MAX_TILES) return 0;
-  int cs = 1;
-  while (cs < max_tiles) cs <<= 1;
-  if (cs > 8 && cudaFuncSetAttribute(resident1d_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                    cudaSuccess) {
+  const void *f = wide ? (const void *)resident1d_kernel<4> : (const void *)resident1d_kernel<1>;
+  if (cs > 8 && cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t c = resident1d_config(cs, 1, nullptr, attr);
+  const cudaLaunchConfig_t c = resident1d_config(cs, 1, wide, nullptr, attr);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, (const void *)resident1d_kernel, &c) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, f, &c) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  return n >= 1 ? cs : 0;
+  return n;
 }
 
-cudaError_t launch_resident1d(int cs, int nprob, const ProbDev *probs, ProbTime *times, const Tables &tb,
+int resident1d_cluster_size(int max_tiles, int nprob, bool *wide)
+{
+  *wide = false;
+  if (max_tiles < 1 || max_tiles > RESIDENT1D_MAX_TILES) return 0;
+  int cs = 1;
+  while (cs < max_tiles) cs <<= 1;
+  if (resident1d_clusters(cs, false) < 1) return 0;
+  // four threads per zone while every problem's cluster runs at once with an SM per CTA
+  *wide = resident1d_clusters(cs, true) >= nprob;
+  return cs;
+}
+
+cudaError_t launch_resident1d(int cs, bool wide, int nprob, const ProbDev *probs, ProbTime *times, const Tables &tb,
                               StateSoA p, StateSoA ph, int nsteps, int *err, cudaStream_t st)
 {
   if (nsteps <= 0 || nprob <= 0) return cudaSuccess;
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t c = resident1d_config(cs, nprob, st, attr);
+  const cudaLaunchConfig_t c = resident1d_config(cs, nprob, wide, st, attr);
   static const TmaTables1d none{};
-  return cudaLaunchKernelEx(&c, resident1d_kernel, probs, times, tb, p, ph, nsteps, err, none);
+  if (wide) return cudaLaunchKernelEx(&c, resident1d_kernel<4>, probs, times, tb, p, ph, nsteps, err, none);
+  return cudaLaunchKernelEx(&c, resident1d_kernel<1>, probs, times, tb, p, ph, nsteps, err, none);
 }
 
 void launch_stage1d(int stage, const ProbDev *probs, ProbTime *times, const Tile *tiles, int ntiles,
