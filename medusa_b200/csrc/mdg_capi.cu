@@ -1595,7 +1595,7 @@ int mdg_eos_given_rex(mdg_eos_table *t, long long n, const double *rho, const do
   if (n > 0 && (!rho || !u || !ye || !temp || !press || !cs || !ent || !gam1))
     return fail(MDG_ERR_INVALID, "null zone array");
   CK(cudaSetDevice(t->device));
-  launch_eos_rex(t->dev(), n, rho, u, ye, temp, press, cs, ent, gam1, t->num_sms, (cudaStream_t)stream);
+  launch_eos_rex(t->dev(), n, rho, u, ye, temp, press, cs, ent, gam1, (cudaStream_t)stream);
   CK(cudaGetLastError());
   return MDG_OK;
 }
@@ -1619,7 +1619,7 @@ int mdg_eos_given_rex_host(mdg_eos_table *t, long long n, const double *rho, con
   for (int k = 0; k < 4 && e == cudaSuccess; k++)
     e = cudaMemcpyAsync(dz[k], hin[k], b, cudaMemcpyHostToDevice, t->stream);
   if (e == cudaSuccess) {
-    launch_eos_rex(t->dev(), n, dz[0], dz[1], dz[2], dz[3], dz[4], dz[5], dz[6], dz[7], t->num_sms, t->stream);
+    launch_eos_rex(t->dev(), n, dz[0], dz[1], dz[2], dz[3], dz[4], dz[5], dz[6], dz[7], t->stream);
     e = cudaGetLastError();
   }
   double *dout[5] = {dz[3], dz[4], dz[5], dz[6], dz[7]};
