@@ -659,7 +659,7 @@ void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, Prob
     shell_mass3_kernel<<<(g.n1 + 127) / 128, 128, 0, st>>>(times, g, sst);
     monopole_profile3_kernel<<<1, 32, 0, st>>>(times, g);
   }
-  const FaceLaunch3 f{{w->nt[0], w->nt[1], w->nt[2]}, {r0, r1}, {l0, l1, l2}, {w->nrun[0], w->nrun[1]},
+  const FaceLaunch3 f{{w->nt[0], w->nt[1], w->nt[2]}, w->num_sms, {r0, r1}, {l0, l1, l2}, {w->nrun[0], w->nrun[1]},
                       {w->nlane[0], w->nlane[1]}, w->nseg, segs, {F0, F1, F2}, own, all0};
   if (mixed) launch_faces3_mixed(stage, f, probs, times, g, sst, st);
   else if (stage == 0) launch_faces3<0, false>(f, probs, times, g, sst, st);

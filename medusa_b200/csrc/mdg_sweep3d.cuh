@@ -50,7 +50,11 @@ constexpr int NT3 = 128;
 #ifndef MDG_F3MINB_MIX
 #define MDG_F3MINB_MIX 7
 #endif
-constexpr int f3_minb(bool mix) { return mix ? MDG_F3MINB_MIX : MDG_F3MINB; }
+// Launches of at most F3MINB_SMALL CTAs per SM are all resident with 96 registers a thread as
+// well, which leaves fewer spills on the chain of one thread's operations: 2-D 400 x 256 blast,
+// 725 CTAs, plain FP64 210 -> 191 us per step, mixed 207 -> 161 us.
+constexpr int F3MINB_SMALL = 5;
+constexpr int f3_minb(bool mix, bool small) { return small ? F3MINB_SMALL : mix ? MDG_F3MINB_MIX : MDG_F3MINB; }
 #ifndef MDG_P3MINB
 #define MDG_P3MINB 8
 #endif
@@ -507,8 +511,8 @@ __device__ __forceinline__ Run3 lane_run(const Run3 *__restrict__ runs, int nrun
 // The RK stage is a run-time argument here (not a template argument as in the other
 // face kernels): both stages then run the same code, which measured faster for stage 1
 // than its own specialisation.
-template <bool MIX>
-__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face0_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+template <bool MIX, bool SMALL>
+__global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face0_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Run3 *__restrict__ runs, int nrun,
                                                      const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, unsigned char *__restrict__ own,
@@ -631,8 +635,8 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX)) face0_kernel(const ProbDev 
 // is then the same for all faces of the run); a thread walks northwards through its
 // column, one new entry and one zone reconstruction per face.  Run3 fields here:
 // r0 = j0, nr = faces, row = i.
-template <bool MIX>
-__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face1_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+template <bool MIX, bool SMALL>
+__global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face1_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Run3 *__restrict__ runs, int nrun,
                                                      const int *__restrict__ first, int nlane, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
@@ -753,8 +757,8 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX)) face1_kernel(const ProbDev 
 // one face.  With one row per CTA the 128 x 64 x 128 grid ran 13274 CTAs at 20 active
 // threads per warp instruction (0.36 ms a stage, plain FP64).
 constexpr int T2 = NT3 - 2;
-template <int STAGE, bool MIX>
-__global__ void __launch_bounds__(NT3, f3_minb(MIX)) face2_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
+template <int STAGE, bool MIX, bool SMALL>
+__global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face2_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
                                                      Grid3 g, const Seg2 *__restrict__ segs, int nseg,
                                                      const int *__restrict__ first, StateSoA s,
                                                      double *__restrict__ flux, const unsigned char *__restrict__ own,
@@ -890,6 +894,7 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX)) face2_kernel(const ProbDev 
 // (mdg_sweep3d_mixed.cu): work lists, fluxes and shock bits as Sweep3 holds them.
 struct FaceLaunch3 {
   int nt[3];                        // CTAs of the three kernels
+  int num_sms;
   const Run3 *runs[2];
   const int *first[3];
   int nrun[2], nlane[2], nseg;
@@ -901,13 +906,16 @@ template <int STAGE, bool MIX>
 inline void launch_faces3(const FaceLaunch3 &f, const ProbDev *probs, ProbTime *times, const Grid3 &g, StateSoA s,
                           cudaStream_t st)
 {
-  face0_kernel<MIX><<<f.nt[0], NT3, 0, st>>>(probs, times, g, f.runs[0], f.nrun[0], f.first[0], f.nlane[0], s, f.F[0],
-                                             f.own, f.all0, STAGE);
-  face1_kernel<MIX><<<f.nt[1], NT3, 0, st>>>(probs, times, g, f.runs[1], f.nrun[1], f.first[1], f.nlane[1], s, f.F[1],
-                                             f.own, f.all0, STAGE);
+  auto small = [&](int k) { return f.nt[k] <= F3MINB_SMALL * f.num_sms; };
+  auto k0 = small(0) ? face0_kernel<MIX, true> : face0_kernel<MIX, false>;
+  auto k1 = small(1) ? face1_kernel<MIX, true> : face1_kernel<MIX, false>;
+  auto k2 = small(2) ? face2_kernel<STAGE, MIX, true> : face2_kernel<STAGE, MIX, false>;
+  k0<<<f.nt[0], NT3, 0, st>>>(probs, times, g, f.runs[0], f.nrun[0], f.first[0], f.nlane[0], s, f.F[0], f.own, f.all0,
+                              STAGE);
+  k1<<<f.nt[1], NT3, 0, st>>>(probs, times, g, f.runs[1], f.nrun[1], f.first[1], f.nlane[1], s, f.F[1], f.own, f.all0,
+                              STAGE);
   if (f.nt[2] > 0)
-    face2_kernel<STAGE, MIX><<<f.nt[2], NT3, 0, st>>>(probs, times, g, f.segs, f.nseg, f.first[2], s, f.F[2], f.own,
-                                                      f.all0);
+    k2<<<f.nt[2], NT3, 0, st>>>(probs, times, g, f.segs, f.nseg, f.first[2], s, f.F[2], f.own, f.all0);
 }
 void launch_faces3_mixed(int stage, const FaceLaunch3 &f, const ProbDev *probs, ProbTime *times, const Grid3 &g,
                          StateSoA s, cudaStream_t st);
