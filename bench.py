@@ -597,7 +597,7 @@ def run_ensemble(args, ctx):
         "precision": "mixed: FP32 reconstruction/limiting/Riemann, FP64 state/fluxes/sources/update/dt",
         "launch": dict(tuned, autotune_ms_per_step=tune_ms),
         # per step and lane: dt, the two stage kernels, the time update
-        "gpu_launches": 4 * K * tuned.get("lanes", 1),
+        "gpu_launches": 3 * K * tuned.get("lanes", 1),   # two stages, time update with the next dt
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "mdg_run_host: upload of all %d initial states (pinned H2D) + %d steps + download of "
@@ -702,7 +702,7 @@ def run_kh(args, ctx):
                    "seq_len": ncell, "parallelism": "replicas" if ctx.world > 1 else "single",
                    "precision": "plain FP64 (reference operation order)",
                    "l2": "inputs larger than L2 (state 2 x 168 MB)"},
-        "gpu_launches": 6 * K,
+        "gpu_launches": 5 * K,
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "upload initial state (pinned H2D) + %d steps + download state (pinned D2H)" % K,
@@ -848,7 +848,7 @@ def run_sedov3d(args, ctx):
                    "precision": "plain FP64 (reference operation order)",
                    "grid": sedov3d_grid_text(pb, args.sedov3d_radius),
                    "l2": "inputs larger than L2 (state 2 x %.0f MB)" % (ncell * 40 / 1e6)},
-        "gpu_launches": 10 * K,
+        "gpu_launches": 9 * K,
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "upload initial state (pinned H2D) + %d steps + download state (pinned D2H)" % K,
@@ -1113,8 +1113,8 @@ def run_sod1d(args, ctx):
         "config": {"workload": "sod_1d_cartesian_1024_to_t0.2_fp64", "global_batch": ctx.world, "seq_len": 1024,
                    "parallelism": "replicas" if ctx.world > 1 else "single",
                    "l2": "resident in L2 (80 KB state): a latency-bound job, timed whole"},
-        # resident: one launch per 256 steps; else dt, two stages and the time update per step
-        "gpu_launches": (nmax + 255) // 256 if resident else 4 * nmax,
+        # resident: one launch per 256 steps; else two stages and the time update per step
+        "gpu_launches": (nmax + 255) // 256 if resident else 3 * nmax,
         "resident_cluster_ctas": resident,
         "time_to_solution_ms": ms, "t": t, "clocks": clocks,
         "accuracy": dict({"l1_rho_vs_exact_riemann": l1}, **ref),

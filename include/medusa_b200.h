@@ -248,7 +248,7 @@ int mdg_write_timers(mdg_solver *s, int prob, const char *path);
  *                    most 16 tiles (2016 zones): 1 (default) = mdg_step runs the whole
  *                    step sequence -- dt rules, both RK stages, time update -- in one launch
  *                    per 256 steps, one thread-block cluster of CTAs per problem (the
- *                    per-phase path launches four dependent kernels per step); 0 = the
+ *                    per-phase path launches three dependent kernels per step); 0 = the
  *                    per-phase launches.  Other solvers ignore it; the results do not
  *                    depend on it.  mdg_resident_cluster reports whether it applies.
  */

