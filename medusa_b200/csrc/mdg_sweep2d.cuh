@@ -412,10 +412,10 @@ ysweep2d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
       for (int v = 0; v < 6; v++) pl[v] = syr[v][t - 1];
       pl[6] = gam;
       const bool hlle = (jx == 0) || (jx == n2) || sflag[t] || sflag[t - 1];
-      if (hlle) {
+      if (!MIX) {
+        riemann_any<1, true, double>(hlle, pl, yl, fg, gc, fy, sig);
+      } else if (hlle) {
         riemann_hlle<1, true, double>(pl, yl, fg, gc, fy, sig);
-      } else if (!MIX) {
-        riemann_hllc<1, true, double>(pl, yl, fg, gc, fy, sig);
       } else {
         float sgf;
         int sb;
