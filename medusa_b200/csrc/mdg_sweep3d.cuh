@@ -155,6 +155,19 @@ __device__ __forceinline__ void load7(const Grid3 &g, const ProbDev &P, const St
   w[6] = P.gam;
 }
 
+// load7 of interior zone c; true when a value is -0 (see pencil0).
+__device__ __forceinline__ bool load7_zone(const ProbDev &P, const StateSoA &s, int64_t c, double *w)
+{
+  bool neg0 = false;
+#pragma unroll
+  for (int v = 0; v < NPRIM; v++) w[v] = s.v[v][c];
+  w[5] = eos_press(P.eos, P.gam, P.Kpoly, w[RHO], w[UU]);
+  w[6] = P.gam;
+#pragma unroll
+  for (int v = 0; v < 6; v++) neg0 = neg0 || (w[v] == 0.0 && signbit(w[v]));
+  return neg0;
+}
+
 // kslopes0 / kslopes1: limited phi slope of row (ii, jj) evaluated at the centroid x2p.
 static __device__ void kslope_point(const Grid3 &g, const ProbDev &P, const StateSoA &s, int ii, int jj, int kk,
                              double x2p, double *pp)
@@ -325,65 +338,50 @@ __device__ __forceinline__ void wave_speeds_g(const double *pl, const double *pr
      / (pl[RHO] * (sl - u_l) - pr[RHO] * (sr - u_r));
 }
 
-// riemann_flux_HLLC (riemann.c:328-499) with per-side Gamma; returns isshock.
+// The wave speeds of a face (riemann_flux_HLLC / HLLE, riemann.c:328-499 / 178-325, with
+// per-side Gamma).
+struct Waves3 { double u_l, u_r, sl, sr, ss, p_s; };
+
+// The HLLC flux from the wave speeds.
 template <int DIR>
-__device__ int hllc3(const double *pl, const double *pr, const FaceGeom<double> &g, double *flux, double &sig)
+__device__ __forceinline__ void hllc3_flux(const double *pl, const double *pr, const FaceGeom<double> &g, Waves3 w,
+                                           double *flux, double &sig)
 {
-  int isshock = 0;
-  if (g.area < 1.0e-16) {
-    sig = 1.0e-200;
-#pragma unroll
-    for (int v = 0; v < NPRIM; v++) flux[v] = 0.0;
-    return isshock;
-  }
   const double sc = g.scale;
-  const double u_l = pl[U1 + DIR] * sc, u_r = pr[U1 + DIR] * sc;
-  double sl, sr, ss, p_s;
-  wave_speeds_g(pl, pr, u_l, u_r, false, sl, sr, ss, p_s, isshock);
-  if (ss > sr) sr = 1.001 * ss;
-  if (ss < sl) sl = 1.001 * ss;
-  sig = tmax(fabs(sl), fabs(sr)) / sc;
-  if (sl > 0.0) { pflux<DIR, false, double>(pl, pl[5], g, flux); return isshock; }
-  if (sr < 0.0) { pflux<DIR, false, double>(pr, pr[5], g, flux); return isshock; }
+  if (w.ss > w.sr) w.sr = 1.001 * w.ss;
+  if (w.ss < w.sl) w.sl = 1.001 * w.ss;
+  sig = tmax(fabs(w.sl), fabs(w.sr)) / sc;
+  if (w.sl > 0.0) { pflux<DIR, false, double>(pl, pl[5], g, flux); return; }
+  if (w.sr < 0.0) { pflux<DIR, false, double>(pr, pr[5], g, flux); return; }
   double u[NPRIM], fx[NPRIM], Us[NPRIM], pk[6];
-  const bool left = ss > 0.0;
+  const bool left = w.ss > 0.0;
 #pragma unroll
   for (int v = 0; v < 6; v++) pk[v] = left ? pl[v] : pr[v];
-  const double sk = left ? sl : sr;
-  const double uk = left ? u_l : u_r;
+  const double sk = left ? w.sl : w.sr;
+  const double uk = left ? w.u_l : w.u_r;
   p_uflux<DIR, false, double>(pk, g, pk[5], u, fx);
-  Us[0] = pk[RHO] * (sk - uk) / (sk - ss);
-  Us[UU] = (u[UU] * (sk - uk) - pk[5] * uk + p_s * ss) / (sk - ss);
+  Us[0] = pk[RHO] * (sk - uk) / (sk - w.ss);
+  Us[UU] = (u[UU] * (sk - uk) - pk[5] * uk + w.p_s * w.ss) / (sk - w.ss);
   Us[U1] = pk[U1]; Us[U2] = pk[U2]; Us[U3] = pk[U3];
-  Us[U1 + DIR] = ss / sc;
+  Us[U1 + DIR] = w.ss / sc;
   const double slr = sk / sc;
   const double vc0 = g.g0 * Us[U1], vc1 = g.g1 * Us[U2], vc2 = g.g2 * Us[U3];
   Us[U1] = vc0 * Us[0]; Us[U2] = vc1 * Us[0]; Us[U3] = vc2 * Us[0];
 #pragma unroll
   for (int v = 0; v < NPRIM; v++) flux[v] = g.area * (fx[v] + slr * (Us[v] - u[v]));
-  return isshock;
 }
 
-// riemann_flux_HLLE (riemann.c:178-325) with per-side Gamma.
+// The HLLE flux from the wave speeds.
 template <int DIR, bool MIX>
-__device__ void hlle3(const double *pl, const double *pr, const FaceGeom<double> &g, double *flux, double &sig)
+__device__ __forceinline__ void hlle3_flux(const double *pl, const double *pr, const FaceGeom<double> &g,
+                                           const Waves3 &w, double *flux, double &sig)
 {
-  if (g.area < 1.0e-16) {
-    sig = 1.0e-200;
-#pragma unroll
-    for (int v = 0; v < NPRIM; v++) flux[v] = 0.0;
-    return;
-  }
   const double sc = g.scale;
-  const double u_l = pl[U1 + DIR] * sc, u_r = pr[U1 + DIR] * sc;
-  double sl, sr, ss, p_s;
-  int isshock;
-  wave_speeds_g(pl, pr, u_l, u_r, true, sl, sr, ss, p_s, isshock);
   double ul[NPRIM], ur[NPRIM], fl[NPRIM], fr[NPRIM];
   p_uflux<DIR, false, double>(pl, g, pl[5], ul, fl);
   p_uflux<DIR, false, double>(pr, g, pr[5], ur, fr);
-  const double cmax = tmax(sr / sc, 0.0);
-  const double cmin = fabs(tmin(sl / sc, 0.0));
+  const double cmax = tmax(w.sr / sc, 0.0);
+  const double cmin = fabs(tmin(w.sl / sc, 0.0));
   sig = tmax(cmax, cmin);
   double num[NPRIM], q[NPRIM];
 #pragma unroll
@@ -391,6 +389,40 @@ __device__ void hlle3(const double *pl, const double *pr, const FaceGeom<double>
   quotients<NPRIM, MIX>(num, cmax + cmin, q);
 #pragma unroll
   for (int v = 0; v < NPRIM; v++) flux[v] = q[v];
+}
+
+// FP64 solve of a face by either solver; returns isshock.  The wave speeds are the same but for
+// a NaN clamp, so the lanes of a warp that take different solvers share them, and the kernels
+// hold them once (instruction fetch was the second stall of face2_kernel): 128 x 64 x 128 blast,
+// plain FP64, 1.37 -> 1.24 ms per step.
+template <int DIR, bool MIX = false>
+__device__ __forceinline__ int riemann3(bool hlle, const double *pl, const double *pr, const FaceGeom<double> &g,
+                                        double *flux, double &sig)
+{
+  if (g.area < 1.0e-16) {
+    sig = 1.0e-200;
+#pragma unroll
+    for (int v = 0; v < NPRIM; v++) flux[v] = 0.0;
+    return 0;
+  }
+  Waves3 w;
+  int isshock = 0;
+  w.u_l = pl[U1 + DIR] * g.scale;
+  w.u_r = pr[U1 + DIR] * g.scale;
+  wave_speeds_g(pl, pr, w.u_l, w.u_r, hlle, w.sl, w.sr, w.ss, w.p_s, isshock);
+  if (hlle) hlle3_flux<DIR, MIX>(pl, pr, g, w, flux, sig);
+  else hllc3_flux<DIR>(pl, pr, g, w, flux, sig);
+  return isshock;
+}
+template <int DIR>
+__device__ __forceinline__ int hllc3(const double *pl, const double *pr, const FaceGeom<double> &g, double *flux, double &sig)
+{
+  return riemann3<DIR>(false, pl, pr, g, flux, sig);
+}
+template <int DIR, bool MIX>
+__device__ __forceinline__ void hlle3(const double *pl, const double *pr, const FaceGeom<double> &g, double *flux, double &sig)
+{
+  riemann3<DIR, MIX>(true, pl, pr, g, flux, sig);
 }
 
 // Face geometry of direction d on row (i, j): area[d], scale[1+d][d], gcov[1+d][0..2].
@@ -534,12 +566,31 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face0_kernel(const P
     const int i0 = t.r0, j = t.row, k = lane - t.l0;
     const int64_t rcs = g.n1 + 2 * NG;
     auto slot = [&](int ii) { return (ii - i0 + 2) % NS; };
-#pragma unroll 1
-    for (int ii = i0 - 2; ii <= i0; ii++) {
+    // The rows of the run stand at the faces' resolution: each is its own pencil entry and is read
+    // directly.  Rows of other levels, ghost rows and zones with a -0 take the general entry,
+    // whose index tables, integer divisions and dependent loads every entry went through before:
+    // 384 x 128 x 256 blast, plain FP64 7.10 -> 6.84 ms per step (6.62 with riemann3), mixed 5.46 -> 5.26 ms.  On
+    // small grids, whose runs are a face or two, the rows beside the run are tested as well
+    // (2-D 400 x 256 mixed 170 -> 162 us; on the large grid the test cost 0.3 ms).  zone_of runs
+    // one row ahead of the loads, so that the row tables' latency is not waited for.
+    const int nj_face = nj_of(g, i0), nk_face = nk_of(g, i0, j);
+    auto zone_of = [&](int ii) -> int64_t {
+      if (!SMALL) return (ii >= i0 && ii < i0 + t.nr && ii < g.n1) ? __ldg(g.cell + rowi(g, ii, j)) + k : -1;
+      if (ii < 0 || ii >= g.n1 || nj_of(g, ii) != nj_face) return -1;
+      const int r = rowi(g, ii, j);
+      return __ldg(g.nk + r) == nk_face ? __ldg(g.cell + r) + k : -1;
+    };
+    int64_t zone = zone_of(i0 - 2);
+    auto entry = [&](int ii, int64_t c) {
       double w[7];
-      pencil0(g, P, s, i0, j, k, ii, w);
+      if (c < 0 || load7_zone(P, s, c, w)) pencil0(g, P, s, i0, j, k, ii, w);
 #pragma unroll
       for (int v = 0; v < 7; v++) win[slot(ii)][v][tid] = w[v];
+    };
+#pragma unroll 1
+    for (int ii = i0 - 2; ii <= i0; ii++) {
+      entry(ii, zone);
+      zone = zone_of(ii + 1);
     }
     {
       // right face values of zone i0-1
@@ -561,12 +612,8 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face0_kernel(const P
     }
 #pragma unroll 1
     for (int i = i0; i < i0 + t.nr; i++) {
-      {
-        double w[7];
-        pencil0(g, P, s, i0, j, k, i + 1, w);
-#pragma unroll
-        for (int v = 0; v < 7; v++) win[slot(i + 1)][v][tid] = w[v];
-      }
+      entry(i + 1, zone);
+      zone = zone_of(i + 2);
       double pl[7], pr[7];
       const int sm = slot(i - 1), s0 = slot(i), sp = slot(i + 1);
       if (MIX) {
@@ -590,7 +637,7 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face0_kernel(const P
       double fl[NPRIM], ss;
       int isshock = -1;
       if (!MIX) {
-        isshock = hllc3<0>(pl, pr, fg, fl, ss);
+        isshock = riemann3<0>(false, pl, pr, fg, fl, ss);
       } else {
         if (pl[6] == P.gam && pr[6] == P.gam) {
           float sig;
@@ -657,12 +704,25 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face1_kernel(const P
     const int64_t cs = g.cols1;
     const int64_t base = g.rc1_base[ilog2(djs(g, i))] + NG;
     auto slot = [&](int jj) { return (jj - j0 + 2) % NS; };
-#pragma unroll 1
-    for (int jj = j0 - 2; jj <= j0; jj++) {
+    // As in face0_kernel: an interior theta row at the faces' phi resolution is its own entry.
+    const int row_i = rowi(g, i, 0), nj_i = nj_of(g, i);
+    const int nk_face = max(nk_of(g, i, j0), nk_of(g, i, j0 - 1));
+    auto zone_of = [&](int jj) -> int64_t {
+      return (jj >= 0 && jj < nj_i && __ldg(g.nk + row_i + jj) == nk_face) ? __ldg(g.cell + row_i + jj) + kk : -1;
+    };
+    int64_t zone = zone_of(j0 - 2);
+    auto entry = [&](int jj, int64_t c) {
       double w[7];
-      pencil1(g, P, s, i, j0, kk, jj, w);
+      if (c < 0) pencil1(g, P, s, i, j0, kk, jj, w);
+      else load7_zone(P, s, c, w);
 #pragma unroll
       for (int v = 0; v < 7; v++) win[slot(jj)][v][tid] = w[v];
+    };
+#pragma unroll 1
+    for (int jj = j0 - 2; jj <= j0; jj++) {
+      const int64_t c = zone;
+      zone = zone_of(jj + 1);
+      entry(jj, c);
     }
     {
       // right face values of zone j0-1
@@ -684,12 +744,8 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face1_kernel(const P
     }
 #pragma unroll 1
     for (int j = j0; j < j0 + t.nr; j++) {
-      {
-        double w[7];
-        pencil1(g, P, s, i, j0, kk, j + 1, w);
-#pragma unroll
-        for (int v = 0; v < 7; v++) win[slot(j + 1)][v][tid] = w[v];
-      }
+      entry(j + 1, zone);
+      zone = zone_of(j + 2);
       double pl[7], pr[7];
       const int sm = slot(j - 1), s0 = slot(j), sp = slot(j + 1);
       if (MIX) {
@@ -719,10 +775,10 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face1_kernel(const P
       const int ij = rowi(g, i, j);
       const FaceGeom<double> fg = face_geom3<1>(g, ij);
       double fl[NPRIM], ss;
-      if (hlle) {
+      if (!MIX) {
+        riemann3<1>(hlle, pl, pr, fg, fl, ss);
+      } else if (hlle) {
         hlle3<1, MIX>(pl, pr, fg, fl, ss);
-      } else if (!MIX) {
-        hllc3<1>(pl, pr, fg, fl, ss);
       } else {
         bool done = false;
         if (pl[6] == P.gam && pr[6] == P.gam) {
@@ -863,10 +919,10 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face2_kernel(const P
     const bool hlle = flag_shock<STAGE>(g, i, j, k, own, all0) || flag_shock<STAGE>(g, i, j, k - 1, own, all0);
     const FaceGeom<double> fg = face_geom3<2>(g, ij);
     double fl[NPRIM], ss;
-    if (hlle) {
+    if (!MIX) {
+      riemann3<2>(hlle, pl, pr, fg, fl, ss);
+    } else if (hlle) {
       hlle3<2, MIX>(pl, pr, fg, fl, ss);
-    } else if (!MIX) {
-      hllc3<2>(pl, pr, fg, fl, ss);
     } else {
       float sig;
       int isshock;
