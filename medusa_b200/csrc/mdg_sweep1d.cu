@@ -371,8 +371,10 @@ int resident1d_cluster_size(int max_tiles, int nprob, bool *wide)
   int cs = 1;
   while (cs < max_tiles) cs <<= 1;
   if (resident1d_clusters(cs, false) < 1) return 0;
-  // four threads per zone while every problem's cluster runs at once with an SM per CTA
-  *wide = resident1d_clusters(cs, true) >= nprob;
+  // four threads per zone, a whole SM per CTA, for up to 16 CTAs: a ninth of the device, so that
+  // several solvers can run beside each other.  (Four solvers of 9 problems of 91-450 zones, 36
+  // CTAs each, took 46 us a step that way and 30 us with one thread per zone.)
+  *wide = cs * nprob <= 16 && resident1d_clusters(cs, true) >= nprob;
   return cs;
 }
 
