@@ -61,31 +61,6 @@ constexpr int TIY2 = MDG_TIY2;    // most rows of a direction-1 tile
 // columns that are swept by the same launches (mdg_sweep2d.cu).
 int tile_rows_2d(int dir, const int *n1, const int *n2, int n, int num_sms);
 
-// Programmatic dependent launches: a kernel launched by launch_dependent may start while the
-// kernel before it in the stream drains, as soon as every CTA of that one has passed
-// allow_dependents; until wait_for_previous returns -- the kernel before has ended and its
-// writes are visible -- it reads only what no kernel writes (tile lists, problem records,
-// tables) and writes nothing.  allow_dependents comes after wait_for_previous, so the order of
-// any two kernels of a chain holds.  Both do nothing in a kernel launched the ordinary way.
-#ifdef __CUDACC__
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename... K, typename... A>
-inline cudaError_t launch_dependent(void (*kernel)(K...), int grid, int block, cudaStream_t st, A... args)
-{
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3((unsigned)grid, 1, 1);
-  c.blockDim = dim3((unsigned)block, 1, 1);
-  c.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = attr;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
-}
-#endif
-
 struct TmaTables1d;
 // Tabulated EOS on the device (mdg_eos_table.cu): the records f[jy][jr][jt] = {e, log p,
 // s, Gamma_1} as two double2 per grid point; grid sizes and bounds as the reference's

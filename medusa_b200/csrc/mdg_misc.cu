@@ -70,8 +70,6 @@ __global__ void finish_kernel(ProbTime *__restrict__ times, int nprob)
 __global__ void finish_next_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times, int nprob, int *err)
 {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  wait_for_previous();
-  allow_dependents();
   if (m >= nprob) return;
   finish_one(times + m);
   dt_finalize_one(probs[m], times + m, err);
@@ -79,7 +77,7 @@ __global__ void finish_next_kernel(const ProbDev *__restrict__ probs, ProbTime *
 
 void launch_finish_next(const ProbDev *probs, ProbTime *times, int nprob, int *err, cudaStream_t st)
 {
-  launch_dependent(finish_next_kernel, (nprob + 127) / 128, 128, st, probs, times, nprob, err);
+  finish_next_kernel<<<(nprob + 127) / 128, 128, 0, st>>>(probs, times, nprob, err);
 }
 
 // monopole_gravity_start/finish (gravity.c:145-425, GR_MONOPOLE=FALSE) of a 1-D problem,

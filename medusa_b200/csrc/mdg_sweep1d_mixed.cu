@@ -296,9 +296,6 @@ stage1d_mixed_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ t
   const int ntiles = use_queue ? q->ntiles : (int)gridDim.x;   // one CTA per tile without the queue
 
   int item;
-  const Tile tile0 = use_queue ? Tile{} : tiles[blockIdx.x];   // while the kernel before drains
-  wait_for_previous();
-  allow_dependents();
   if (use_queue) {
     // the other stage's counter is idle while this kernel runs: reset it for its next launch
     if (blockIdx.x == 0 && t == 0) q->head[1 - STAGE] = 0u;
@@ -310,7 +307,7 @@ stage1d_mixed_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ t
   }
 
   while (item < ntiles) {
-    const Tile tile = use_queue ? tiles[item] : tile0;
+    const Tile tile = tiles[item];
     if (times[tile.prob].done) {       // past tmax: the time loop has ended (CTA-uniform)
       if (!use_queue) break;
       __syncthreads();                  // every thread has read the current s_item
@@ -479,13 +476,10 @@ static void launch_mixed_nt(int stage, int grid, bool use_queue, const ProbDev *
                             const Tile *tiles, WorkQueue *q, const Tables &tb, StateSoA sst, StateSoA sn,
                             StateSoA out, cudaStream_t st)
 {
-  auto kernel = stage == 0 ? stage1d_mixed_kernel<NT, 0, TAB> : stage1d_mixed_kernel<NT, 1, TAB>;
-  // a grid of up to about a wave starts beside the end of the kernel before it: 16 to 24 small
-  // problems 17.9 -> 15.8 and 17.1 -> 15.9 us per step; a large one has nothing to gain
-  if (grid <= 1024)
-    launch_dependent(kernel, grid, NT, st, probs, times, tiles, q, use_queue, tb, sst, sn, out);
+  if (stage == 0)
+    stage1d_mixed_kernel<NT, 0, TAB><<<grid, NT, 0, st>>>(probs, times, tiles, q, use_queue, tb, sst, sn, out);
   else
-    kernel<<<grid, NT, 0, st>>>(probs, times, tiles, q, use_queue, tb, sst, sn, out);
+    stage1d_mixed_kernel<NT, 1, TAB><<<grid, NT, 0, st>>>(probs, times, tiles, q, use_queue, tb, sst, sn, out);
 }
 
 template <bool TAB>
