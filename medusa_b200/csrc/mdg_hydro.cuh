@@ -126,9 +126,8 @@ __device__ __forceinline__ GamConst<T> gam_const(T G)
 // Quotient and square root of the wave-speed estimate.  FP64: the operators (correctly rounded).
 // FP32: the approximate reciprocal (reciprocal square root) and one correction by the exact
 // remainder, a Newton step: within half an ulp and a little, as the rounded operators for the
-// purposes of an FP32 estimate, without their range checks and calls (a zero or infinite
-// divisor gives NaN, where the operator gives an infinity or zero).  The 1-D mixed sweep's
-// fast-math translation unit keeps its approximate operators.
+// purposes of an FP32 estimate (a zero or infinite divisor gives NaN, where the operator gives
+// an infinity or zero).  The 1-D mixed sweep's fast-math translation unit keeps its approximate operators.
 __device__ __forceinline__ double quot(double a, double b) { return a / b; }
 __device__ __forceinline__ double root(double x) { return sqrt(x); }
 __device__ __forceinline__ float quot(float a, float b)

@@ -88,9 +88,8 @@ MDG_HD MDG_INLINE void para_recon_zone(T am_v, T a, T ap_v, const G &g, T &al, T
 // corrected twice by its remainder a - b q, which a fused multiply-add forms exactly
 // (Markstein, IBM J. Res. Dev. 34, 1990: with y the rounded reciprocal and q within one
 // ulp, q + (a - b q) y rounds to the quotient; the first correction puts q there).  Five
-// operations without a branch, where the division operator takes a reciprocal seed, its
-// refinement and a range check with a call behind it.  The caller keeps a and b where no
-// step over- or underflows (recon_in_range).
+// operations without a branch.  The caller keeps a and b where no step over- or underflows
+// (recon_in_range).
 MDG_HD MDG_INLINE double div_by(double a, double b, double y)
 {
   double q = a * y;

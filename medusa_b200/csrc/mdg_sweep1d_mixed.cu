@@ -57,11 +57,9 @@ __device__ __noinline__ float face_fp64(const double *c, int cs, const double *r
 }
 
 // 1/b and 1/sqrt(b) of normal positive FP64 numbers to about an ulp: the approximate instruction
-// (20 bits) and two Newton steps, without the range check, the call and the last-place
-// completion of the operators (6 and 9 instructions for about 18 and 30).  Each stage of a zone
-// took a dozen FP64 divisions, whose last places this sweep's results are not pinned to; with
-// the dt limits divided once per tile, the 2048-problem ensemble went from 0.482 to 0.441 ms
-// per step (errors against 64 bits unchanged: density 3.2e-8 before, 2.7e-8 after 40 steps).
+// (20 bits) and two Newton steps.  Each stage of a zone took a dozen FP64 divisions, whose last
+// places this sweep's results are not pinned to; with the dt limits divided once per tile, the
+// 2048-problem ensemble went from 0.482 to 0.441 ms per step (errors against 64 bits unchanged: density 3.2e-8 before, 2.7e-8 after 40 steps).
 __device__ __forceinline__ double rcp64(double b)
 {
   double y;
