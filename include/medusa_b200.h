@@ -249,8 +249,10 @@ int mdg_write_timers(mdg_solver *s, int prob, const char *path);
  *                    step sequence -- dt rules, both RK stages, time update -- in one launch
  *                    per 256 steps, one thread-block cluster of CTAs per problem (the
  *                    per-phase path launches three dependent kernels per step); 0 = the
- *                    per-phase launches.  Other solvers ignore it; the results do not
- *                    depend on it.  mdg_resident_cluster reports whether it applies.
+ *                    per-phase launches.  A cluster starts when all its CTAs fit at once in
+ *                    one GPC, and where a solver has at most 16 CTAs each takes a whole SM:
+ *                    a program that keeps a kernel of its own running sets it to 0.  Other
+ *                    solvers ignore it; the results do not depend on it.  mdg_resident_cluster reports whether it applies.
  */
 #define MDG_MAX_LANES 4
 typedef struct mdg_launch_config {
@@ -308,6 +310,8 @@ int mdg_conserved_totals(mdg_solver *s, double *mass, double *energy);
  *   - no call can be captured into a CUDA graph: each waits on its stream before it
  *     returns (the host tables must outlive their copies);
  *   - all calls share the array: calls whose work overlaps on the GPU race;
+ *   - the work is queued as ordinary launches, CTAs of 128 threads that run one by one as
+ *     they fit: it makes progress beside a kernel of the caller's that does not end;
  *   - the array keeps the last call's contents; each call re-initialises what it uses;
  *   - the tables are built in one process-wide host buffer under a lock, so calls from
  *     several host threads wait for each other while their tables are copied.

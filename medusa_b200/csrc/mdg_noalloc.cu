@@ -200,15 +200,11 @@ extern "C" int mdg_advance_1d_noalloc(const mdg_problem_desc *desc, const double
 
   launch_reset_time(times, 0, st);
   launch_initial_estimate_one(probs, times, 0, n1, tb, S, st);
-  // the resident stepper where the problem fits a thread-block cluster, else four launches a
-  // step (the same bits): 20 steps of 200 zones 0.88 -> 0.75 ms a call
-  bool wide = false;
-  const int cs = resident1d_cluster_size(ntiles, 1, &wide);
-  for (int k = 0; k < nsteps && cs > 0; k += RESIDENT_STEPS) {
-    const int n = nsteps - k < RESIDENT_STEPS ? nsteps - k : RESIDENT_STEPS;
-    CKN(launch_resident1d(cs, wide, 1, probs, times, tb, S, PH, n, err, st));
-  }
-  for (int k = 0; k < nsteps && cs == 0; k++) {
+  // Three launches a step, each of CTAs that run one by one wherever 128 threads fit.  The
+  // resident stepper's clusters (20 steps of 200 zones 0.64 ms a call for 0.82 ms) start only
+  // when all their CTAs fit at once, which beside a caller's own long-running kernel may be
+  // never; mdg_step's callers can turn it off, this call's cannot.
+  for (int k = 0; k < nsteps; k++) {
     if (k == 0) launch_dt_finalize(probs, times, 1, err, st);
     launch_stage1d(0, probs, times, tiles, ntiles, tb, S, S, PH, st);
     launch_stage1d(1, probs, times, tiles, ntiles, tb, PH, S, S, st);

@@ -22,6 +22,7 @@ import pytest
 from medusa_b200 import problems as P
 from medusa_b200 import solver as S
 from oracle import pyoracle
+from tests import _device
 from tests._cases import field_rel_err, pointwise_rel_err
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +134,32 @@ def test_noalloc_rejects_problems_beyond_the_scratch():
     dummy = ctypes.c_double(0.0)
     rc = f(ctypes.byref(desc), ctypes.addressof(dummy), ctypes.addressof(dummy), 1, None, None, None)
     assert rc == 6   # MDG_ERR_OUTOFMEM: does not fit the fixed scratch
+
+
+@pytest.mark.parametrize("n1", [200, 2016, 2017, 8192])
+def test_noalloc_sizes(n1):
+    """A few tiles, 16 full ones (where the allocating path's one-launch stepper ends), one
+    zone more, and the largest problem."""
+    _check_against_both(P.sod(n1), 6)
+
+
+@pytest.mark.parametrize("left,smem", [(0, 120 << 10), (1, 220 << 10)])
+def test_noalloc_makes_progress_beside_a_long_kernel(left, smem):
+    """A caller's kernel holds every SM but `left` for half a second (with less than all of an
+    SM's shared memory where it holds them all): the call returns while that still runs."""
+    import torch
+    pb = P.sod(2016)
+    want = _with_noalloc_abi(pb, 3)            # (and everything is loaded)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    f, desc = _noalloc_fn(), S.desc_of(pb)
+    d = torch.from_numpy(np.ascontiguousarray(pb.ic.T)).to("cuda")
+    with _device.Hold(1, 32, smem, 1):         # (the helper is loaded too)
+        pass
+    torch.cuda.synchronize()
+    with _device.Hold(sms - left, 32, smem, 500) as hold:
+        assert hold.running()
+        assert f(ctypes.byref(desc), d.data_ptr(), d.data_ptr(), 3, torch.cuda.current_stream().cuda_stream, None,
+                 None) == 0
+        beside = hold.running()
+    assert beside
+    assert np.array_equal(d.cpu().numpy().T, want[0])
