@@ -38,7 +38,11 @@ extern "C" void *hold_start(int sms, int threads, int smem, int ms)
   bool ok = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming) == cudaSuccess &&
             cudaMallocHost(&h->started, sizeof(unsigned int)) == cudaSuccess &&
-            cudaFuncSetAttribute(hold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+            cudaFuncSetAttribute(hold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+            // (an SM keeps its shared-memory carve-out while CTAs run on it: the largest, so that
+            // what these leave is there for others)
+            cudaFuncSetAttribute(hold_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared) == cudaSuccess;
   if (ok) {
     *h->started = 0;
     hold_kernel<<<sms, threads, smem, h->st>>>(h->started, ns, 4ll * ms * 1000);
