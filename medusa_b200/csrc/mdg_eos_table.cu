@@ -23,8 +23,9 @@
 
 namespace mdg {
 
-// 256 threads, 4 CTAs per SM (64 registers), a thread per zone: 4 M zones with warm guesses on a
-// B200 0.433 -> 0.385 ms; 0.41-0.51 ms with 64 or 128 threads or more CTAs and fewer registers.
+// 256 threads, 4 CTAs per SM (64 registers), a thread per zone: 4 M zones on a B200, L2 flushed
+// between calls (8 CTAs of 256 threads per SM in a grid-stride loop before): guesses from the last
+// step 0.447 -> 0.426 ms, a row too high 0.444 -> 0.424, a row too low 0.506 -> 0.490.
 constexpr int EOS_NT = 256;
 
 __global__ void __launch_bounds__(EOS_NT, 4)
@@ -86,20 +87,22 @@ eos_rex_kernel(EosTableDev d, long long n, const double *__restrict__ rho, const
       return e;
     };
 
-    // the guess's row and the next one first, all eight sectors at once: a guess from the
-    // last step brackets the energy, and the search below ends without another load
-    double elo = energy(jt), ehi = energy(jt + 1);
-    if (!(elo < e_eos || jt == 1)) {
-      do {
-        ehi = elo;
-        jt = jt - 1;
-        elo = energy(jt);
-      } while (!(elo < e_eos || jt == 1));
-    } else {
-      while (!(ehi > e_eos || jt == nt - 1)) {
+    // (Both rows read at once are faster for guesses from the last step, 4 M zones 404 for 426 us,
+    // but a guess that lies a row or two too high has then read a row in vain: 469 for 424 us and
+    // 522 for 490 us.)
+    double elo, ehi = -1e99;
+    while (true) {
+      elo = energy(jt);
+      if (elo < e_eos || jt == 1) break;
+      ehi = elo;
+      jt = jt - 1;
+    }
+    if (ehi < -1e98) {
+      while (true) {
+        ehi = energy(jt + 1);
+        if (ehi > e_eos || jt == nt - 1) break;
         elo = ehi;
         jt = jt + 1;
-        ehi = energy(jt + 1);
       }
     }
     const double tlo = t1 + (jt - 1) * dt;

@@ -72,3 +72,17 @@ def test_gpu_eos_device_path_equals_host_path():
     assert np.array_equal(dev[3].cpu().numpy(), host[0])
     for k in range(4):
         assert np.array_equal(outs[k].cpu().numpy(), host[k + 1])
+
+
+def test_gpu_eos_results_do_not_depend_on_the_guess():
+    """Guesses in the right row, one and two rows off either way and at both ends of the table
+    bracket the same rows: the same bits."""
+    g = ET.EosGrid(nrec=12, ny=9, nr=40, nt=50)
+    tab = ET.synthetic_table(g)
+    rho, u, ye, tg = ET.synthetic_zones(g, 4000, seed=5, table=tab)
+    row = 10.0 ** ((g.t2 - g.t1) / (g.nt - 1))
+    with ET.EosTable(tab, g) as t:
+        want = t.given_rex(rho, u, ye, tg)
+        for guess in [want[0] * row ** k for k in (-2, -1, 0, 1, 2)] + [np.full_like(tg, 10.0 ** x) for x in (g.t1, g.t2)]:
+            got = t.given_rex(rho, u, ye, guess)
+            assert all(np.array_equal(a, b) for a, b in zip(got, want))
