@@ -56,25 +56,6 @@ __device__ __noinline__ float face_fp64(const double *c, int cs, const double *r
   return (float)sig64;
 }
 
-// 1/b and 1/sqrt(b) of normal positive FP64 numbers to about an ulp: the approximate instruction
-// (20 bits) and two Newton steps.  Each stage of a zone took a dozen FP64 divisions, whose last
-// places this sweep's results are not pinned to; with the dt limits divided once per tile, the
-// 2048-problem ensemble went from 0.482 to 0.441 ms per step (errors against 64 bits unchanged: density 3.2e-8 before, 2.7e-8 after 40 steps).
-__device__ __forceinline__ double rcp64(double b)
-{
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  y = fma(y, fma(-b, y, 1.0), y);
-  return fma(y, fma(-b, y, 1.0), y);
-}
-__device__ __forceinline__ double rsqrt64(double b)
-{
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  y = fma(0.5 * y, fma(-b * y, y, 1.0), y);
-  return fma(0.5 * y, fma(-b * y, y, 1.0), y);
-}
-
 // 1-D geometry in closed form, in FP64.  On the uniform-radius spherical grid (r = x,
 // dr/dx = 1) every quantity of metric_spherical_general.c is a polynomial integral over the
 // zone's edge radii a < b times an angular constant (ProbDev::gk_*); written with the
@@ -169,14 +150,7 @@ __device__ __forceinline__ double dt_source_control_1div(const double *p, const 
   const double momterm = p[U1] * s[U1] + p[U2] * s[U2] + p[U3] * s[U3];
   const double n2 = 100 * alpha * p[UU], d2 = fabs(fabs(s[1]) - fabs(momterm)) + 1.0e-16;
   if (n2 * den < num * d2) { num = n2; den = d2; }
-  return fmin(1.0e100, num * rcp64(den));   // den >= 1e-16
-}
-
-// sqrt(gp / rho), gp = Gamma p; 0 for gp = 0, NaN below it, as sqrt
-__device__ __forceinline__ double sound_speed(double gp, double rho)
-{
-  const double x = gp * rho;
-  return (x == 0.0) ? 0.0 : gp * rsqrt64(x);
+  return fmin(1.0e100, num * rcp64(den));   // den >= 1e-16; infinite: the update is, and is flagged
 }
 
 // Face geometry of a problem on a non-uniform coordinate map (the Romberg tables).
