@@ -271,11 +271,23 @@ int mdg_set_launch_config(mdg_solver *s, const mdg_launch_config *cfg);
  * queues ceil(n / 256) kernel launches. */
 int mdg_resident_cluster(mdg_solver *s, int *ctas);
 
+/* The work lists of a dendritic solver fixed by hand (to measure the size rules, and for
+ * tests; the results do not depend on the run length, and in plain FP64 not on the kernels
+ * either; in mixed precision the two kernels round differently): runs of exactly run_length faces, 1..64, whatever
+ * the grid's size (0: mdg_launch_config::run_length at most, by the grid's size; so again
+ * after that is changed); small_launch 1 or 0 = the face kernels with the registers of small
+ * launches or of large ones (-1: by the grid's size).  mdg_get_run_shape: the run length
+ * in use, and bit k set where face kernel k is the small launches'.  MDG_ERR_NOTIMPL for other
+ * solvers. */
+int mdg_set_run_shape(mdg_solver *s, int run_length, int small_launch);
+int mdg_get_run_shape(mdg_solver *s, int *run_length, int *small_launch);
+
 /* Time every admissible launch shape over trial_steps steps of the solver's own
  * problems, keep the fastest and restore the state, times and error flag as they were:
  * (threads, ctas_per_sm) of the batched 1-D mixed sweep and then its lanes (1, 2, 4) with
- * the best of those, run_length (4, 8, 16, 32) of a dendritic-grid solver of either
- * precision.  best/ms_per_step may be NULL.
+ * the best of those, the run length of a dendritic-grid solver of either precision: the
+ * one its grid's size gives (reported as run_length 16) and 4, 8, 16 and 32 as they are,
+ * kept until run_length is changed.  best/ms_per_step may be NULL.
  * MDG_ERR_NOTIMPL for the FP64 1-D and 2-D Cartesian solvers, whose shapes are fixed. */
 int mdg_autotune(mdg_solver *s, int trial_steps, mdg_launch_config *best, double *ms_per_step);
 

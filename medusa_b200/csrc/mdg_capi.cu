@@ -1093,7 +1093,7 @@ int mdg_set_launch_config(mdg_solver *s, const mdg_launch_config *cfg)
   CK(cudaStreamSynchronize(s->stream));
   if (s->ndim == 3 && cfg->run_length != s->cfg.run_length) {
     std::string why;
-    const int rc = sweep3_set_run_length(s->s3, cfg->run_length, why);
+    const int rc = sweep3_set_run_length(s->s3, cfg->run_length, 0, why);
     if (rc != MDG_OK) return fail(rc, "run_length: " + why);
     drop_graph(s);
   }
@@ -1107,6 +1107,31 @@ int mdg_set_launch_config(mdg_solver *s, const mdg_launch_config *cfg)
   if (reshape || cfg->ctas_per_sm != s->cfg.ctas_per_sm || cfg->steps_per_graph != s->cfg.steps_per_graph)
     drop_graph(s);
   s->cfg = *cfg;
+  return MDG_OK;
+}
+
+int mdg_set_run_shape(mdg_solver *s, int run_length, int small_launch)
+{
+  if (!s) return fail(MDG_ERR_INVALID, "solver");
+  if (s->ndim != 3) return fail(MDG_ERR_NOTIMPL, "only the dendritic sweeps walk runs of faces");
+  if (run_length < 0 || run_length > 64) return fail(MDG_ERR_INVALID, "run_length out of [0, 64]");
+  if (small_launch < -1 || small_launch > 1) return fail(MDG_ERR_INVALID, "small_launch out of [-1, 1]");
+  CK(cudaSetDevice(s->device));
+  CK(cudaStreamSynchronize(s->stream));
+  std::string why;
+  const int rc = sweep3_set_run_length(s->s3, s->cfg.run_length, run_length, why);
+  if (rc != MDG_OK) return fail(rc, "run_length: " + why);
+  sweep3_set_small(s->s3, small_launch);
+  drop_graph(s);
+  return MDG_OK;
+}
+
+int mdg_get_run_shape(mdg_solver *s, int *run_length, int *small_launch)
+{
+  if (!s || !run_length || !small_launch) return fail(MDG_ERR_INVALID, "solver/run_length/small_launch");
+  if (s->ndim != 3) return fail(MDG_ERR_NOTIMPL, "only the dendritic sweeps walk runs of faces");
+  int exact = 0;
+  sweep3_run_shape(s->s3, &exact, run_length, small_launch);
   return MDG_OK;
 }
 
@@ -1133,8 +1158,23 @@ int mdg_autotune(mdg_solver *s, int trial_steps, mdg_launch_config *best, double
     CK(cudaStreamSynchronize(s->stream));
     return MDG_OK;
   };
-  const mdg_launch_config orig = s->cfg;
-  mdg_launch_config bestc = orig;
+  // a candidate: the launch shape and, for a dendritic sweep, the run length as it is (0: by the
+  // grid's size, at most the shape's)
+  struct Cand { mdg_launch_config c; int exact; };
+  auto apply = [&](const Cand &q) -> int {
+    int r = mdg_set_launch_config(s, &q.c);
+    if (r == MDG_OK && dendritic) {
+      std::string why;
+      r = sweep3_set_run_length(s->s3, q.c.run_length, q.exact, why);
+      if (r != MDG_OK) return fail(r, "run_length: " + why);
+      drop_graph(s);
+    }
+    return r;
+  };
+  int used = 0, small = 0;
+  Cand orig{s->cfg, 0};
+  if (dendritic) sweep3_run_shape(s->s3, &orig.exact, &used, &small);
+  Cand bestc = orig;
   double bestms = 1.0e300;
   do {
     if (cudaMalloc(&bk, sbytes) != cudaSuccess || cudaMalloc(&bt, sizeof(ProbTime) * s->nprob) != cudaSuccess) {
@@ -1148,24 +1188,28 @@ int mdg_autotune(mdg_solver *s, int trial_steps, mdg_launch_config *best, double
       rc = fail(MDG_ERR_CUDA, "autotune: set-up");
       break;
     }
-    // candidate shapes: (threads, ctas_per_sm) of the mixed 1-D sweep, or the run length
-    // of a dendritic sweep
-    std::vector<mdg_launch_config> cand;
-    const int k = orig.steps_per_graph;
+    // candidate shapes: (threads, ctas_per_sm) of the mixed 1-D sweep; the run length of a
+    // dendritic sweep, first the one its grid's size gives, then others
+    std::vector<Cand> cand;
+    const mdg_launch_config &o = orig.c;
+    const int k = o.steps_per_graph;
     if (dendritic) {
-      for (int len : {4, 8, 16, 32})
-        cand.push_back(mdg_launch_config{orig.threads, orig.ctas_per_sm, k, len, 1, orig.resident});
+      cand.push_back(Cand{{o.threads, o.ctas_per_sm, k, 16, 1, o.resident}, 0});
+      for (int len : {4, 8, 16, 32}) cand.push_back(Cand{{o.threads, o.ctas_per_sm, k, len, 1, o.resident}, len});
     } else {
       for (int nt : {64, 128, 256}) {
         const int occ = mixed_max_ctas_per_sm(nt);
         for (int c : {0, 1, 2, 3, 4, 6, 8, 12, 16})
-          if (c <= occ) cand.push_back(mdg_launch_config{nt, c, k, orig.run_length, 1, orig.resident});
+          if (c <= occ) cand.push_back(Cand{{nt, c, k, o.run_length, 1, o.resident}, 0});
       }
     }
     const int steps = (k > 0) ? ((trial_steps + k - 1) / k) * k : trial_steps;
     // one trial: the state restored, a warm-up (and graph capture), then `steps` timed steps
-    auto trial = [&](const mdg_launch_config &c) -> int {
-      int r = mdg_set_launch_config(s, &c);
+    int by_size = 0;   // run length of the first dendritic candidate
+    auto trial = [&](const Cand &c) -> int {
+      if (c.exact && c.exact == by_size) return MDG_OK;   // tried already
+      int r = apply(c);
+      if (dendritic && !c.exact) sweep3_run_shape(s->s3, &used, &by_size, &small);
       if (r == MDG_OK) r = restore();
       if (r == MDG_OK) r = mdg_step(s, k > 0 ? k : 1);
       if (r != MDG_OK) return r;
@@ -1183,16 +1227,16 @@ int mdg_autotune(mdg_solver *s, int trial_steps, mdg_launch_config *best, double
     for (size_t ci = 0; ci < cand.size() && rc == MDG_OK; ci++) rc = trial(cand[ci]);
     // the mixed 1-D sweep: lanes with the best (threads, ctas_per_sm)
     if (!dendritic) {
-      const mdg_launch_config shape = bestc;
+      const Cand shape = bestc;
       for (int nl : {2, 4}) {
         if (rc != MDG_OK) break;
-        mdg_launch_config c = shape;
-        c.lanes = nl;
+        Cand c = shape;
+        c.c.lanes = nl;
         rc = trial(c);
       }
     }
-    if (rc == MDG_OK) rc = mdg_set_launch_config(s, &bestc);
-    else mdg_set_launch_config(s, &orig);
+    if (rc == MDG_OK) rc = apply(bestc);
+    else apply(orig);
     const int rc2 = restore();
     if (rc == MDG_OK) rc = rc2;
   } while (0);
@@ -1201,7 +1245,7 @@ int mdg_autotune(mdg_solver *s, int trial_steps, mdg_launch_config *best, double
   cudaFree(bk);
   cudaFree(bt);
   if (rc != MDG_OK) return rc;
-  if (best) *best = bestc;
+  if (best) *best = bestc.c;
   if (ms_per_step) *ms_per_step = bestms;
   return MDG_OK;
 }

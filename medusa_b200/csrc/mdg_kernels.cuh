@@ -115,7 +115,9 @@ void sweep3_destroy(Sweep3 *w);
 int64_t sweep3_ncell(const Sweep3 *w);
 int64_t sweep3_bytes(const Sweep3 *w);   // device memory of the grid tables, face fluxes and bits
 // Faces per work item of the radial and theta run kernels (1..64); rebuilds the work lists.
-int sweep3_set_run_length(Sweep3 *w, int run_length, std::string &why);
+int sweep3_set_run_length(Sweep3 *w, int run_length, int exact, std::string &why);
+void sweep3_set_small(Sweep3 *w, int small);
+void sweep3_run_shape(const Sweep3 *w, int *exact, int *used, int *small);
 void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, ProbTime *times,
                     StateSoA stage_state, StateSoA state_n, StateSoA out, cudaStream_t st);
 void launch_initial_estimate3(Sweep3 *w, const ProbDev *probs, ProbTime *times, StateSoA s, cudaStream_t st);

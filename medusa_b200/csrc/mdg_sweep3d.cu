@@ -296,7 +296,11 @@ struct Sweep3 {
   size_t runs_cap = 0;             // ints d_runs holds
   size_t run_off[4] = {0, 0, 0, 0};
   int nrun[2] = {0, 0}, nlane[2] = {0, 0};
-  int run_len = RUN0;
+  int run_len = RUN0;              // longest run asked for
+  int run_exact = 0;               // a length fixed by hand, whatever the grid's size (0: fitting_run)
+  int run_used = 0;                // the length the lists are cut to
+  bool small_rule[3] = {false, false, false};   // face kernel k's launch is a small one (small_by_size)
+  int small = -1;                  // the small launches' kernels: by that rule (-1), never, always
   int num_sms = 0;
   // the row structure the run lists are cut from (a copy of the host grid's)
   int n1 = 0, n2 = 0, n3 = 0;
@@ -383,7 +387,6 @@ static void build_runs(const Sweep3 &w, int dir, int run_len, RunList &out)
 {
   std::vector<Run3> runs;
   std::vector<int> cnt;
-  run_len = fitting_run(w, run_len);
   cut_runs(w, dir, run_len, runs, cnt);
   // long runs first (the tail of the launch is made of short ones), neighbouring rows in
   // neighbouring lanes: direction 0 by first face then theta row, direction 1 likewise
@@ -430,14 +433,21 @@ static void build_segs(const Sweep3 &w, std::vector<Seg2> &segs, std::vector<int
   }
 }
 
-// Both run lists for runs of at most run_len faces, into one device allocation.
-static cudaError_t upload_runs(Sweep3 *w, int run_len)
+// Both run lists for runs of at most run_len faces (exact != 0: of that many, else shorter ones
+// where the grid is small), into one device allocation.
+static cudaError_t upload_runs(Sweep3 *w, int run_len, int exact)
 {
+  const int used = exact ? exact : fitting_run(*w, run_len);
+  if (used == w->run_used) {
+    w->run_len = run_len;
+    w->run_exact = exact;
+    return cudaSuccess;
+  }
   RunList l[2];
   std::vector<int> all;
   size_t off[4];
   for (int d = 0; d < 2; d++) {
-    build_runs(*w, d, run_len, l[d]);
+    build_runs(*w, d, used, l[d]);
     off[d] = all.size();
     const int *r = reinterpret_cast<const int *>(l[d].runs.data());
     all.insert(all.end(), r, r + sizeof(Run3) / sizeof(int) * l[d].runs.size());
@@ -464,19 +474,40 @@ static cudaError_t upload_runs(Sweep3 *w, int run_len)
     w->nlane[d] = l[d].nlane;
   }
   w->run_len = run_len;
+  w->run_exact = exact;
+  w->run_used = used;
   return cudaSuccess;
 }
 
-int sweep3_set_run_length(Sweep3 *w, int run_length, std::string &why)
+int sweep3_set_run_length(Sweep3 *w, int run_length, int exact, std::string &why)
 {
   if (run_length < 1 || run_length > 64) { why = "run_length out of [1, 64]"; return MDG_ERR_INVALID; }
-  if (run_length == w->run_len) return MDG_OK;
-  const cudaError_t e = upload_runs(w, run_length);
+  if (exact < 0 || exact > 64) { why = "exact run length out of [0, 64]"; return MDG_ERR_INVALID; }
+  const cudaError_t e = upload_runs(w, run_length, exact);
   if (e != cudaSuccess) {
     why = cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? MDG_ERR_OUTOFMEM : MDG_ERR_CUDA;
   }
   return MDG_OK;
+}
+void sweep3_set_small(Sweep3 *w, int small) { w->small = small; }
+static bool small_launch(const Sweep3 &w, int k)
+{
+  return w.small >= 0 ? w.small == 1 : w.small_rule[k];
+}
+// Which launches are small is settled once, with the run length that the grid's size gives: the two
+// variants of a mixed kernel contract differently, and the results are not to depend on the run
+// length that is set later.
+static void small_by_size(Sweep3 *w)
+{
+  for (int k = 0; k < 3; k++) w->small_rule[k] = w->nt[k] <= F3MINB_SMALL * w->num_sms;
+}
+void sweep3_run_shape(const Sweep3 *w, int *exact, int *used, int *small)
+{
+  *exact = w->run_exact;
+  *used = w->run_used;
+  *small = 0;
+  for (int k = 0; k < 3; k++) *small |= small_launch(*w, k) ? 1 << k : 0;
 }
 
 int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
@@ -625,8 +656,9 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     e = cudaMemcpy(w->d_seg, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail3(e);
   }
-  e = upload_runs(w, RUN0);
+  e = upload_runs(w, RUN0, 0);
   if (e != cudaSuccess) return fail3(e);
+  small_by_size(w);
   *out = w;
   return MDG_OK;
 }
@@ -659,7 +691,7 @@ void launch_stage3d(int stage, bool mixed, Sweep3 *w, const ProbDev *probs, Prob
     shell_mass3_kernel<<<(g.n1 + 127) / 128, 128, 0, st>>>(times, g, sst);
     monopole_profile3_kernel<<<1, 32, 0, st>>>(times, g);
   }
-  const FaceLaunch3 f{{w->nt[0], w->nt[1], w->nt[2]}, w->num_sms, {r0, r1}, {l0, l1, l2}, {w->nrun[0], w->nrun[1]},
+  const FaceLaunch3 f{{w->nt[0], w->nt[1], w->nt[2]}, {small_launch(*w, 0), small_launch(*w, 1), small_launch(*w, 2)}, {r0, r1}, {l0, l1, l2}, {w->nrun[0], w->nrun[1]},
                       {w->nlane[0], w->nlane[1]}, w->nseg, segs, {F0, F1, F2}, own, all0};
   if (mixed) launch_faces3_mixed(stage, f, probs, times, g, sst, st);
   else if (stage == 0) launch_faces3<0, false>(f, probs, times, g, sst, st);

@@ -950,7 +950,7 @@ __global__ void __launch_bounds__(NT3, f3_minb(MIX, SMALL)) face2_kernel(const P
 // (mdg_sweep3d_mixed.cu): work lists, fluxes and shock bits as Sweep3 holds them.
 struct FaceLaunch3 {
   int nt[3];                        // CTAs of the three kernels
-  int num_sms;
+  bool small[3];                    // at most F3MINB_SMALL CTAs per SM
   const Run3 *runs[2];
   const int *first[3];
   int nrun[2], nlane[2], nseg;
@@ -962,10 +962,9 @@ template <int STAGE, bool MIX>
 inline void launch_faces3(const FaceLaunch3 &f, const ProbDev *probs, ProbTime *times, const Grid3 &g, StateSoA s,
                           cudaStream_t st)
 {
-  auto small = [&](int k) { return f.nt[k] <= F3MINB_SMALL * f.num_sms; };
-  auto k0 = small(0) ? face0_kernel<MIX, true> : face0_kernel<MIX, false>;
-  auto k1 = small(1) ? face1_kernel<MIX, true> : face1_kernel<MIX, false>;
-  auto k2 = small(2) ? face2_kernel<STAGE, MIX, true> : face2_kernel<STAGE, MIX, false>;
+  auto k0 = f.small[0] ? face0_kernel<MIX, true> : face0_kernel<MIX, false>;
+  auto k1 = f.small[1] ? face1_kernel<MIX, true> : face1_kernel<MIX, false>;
+  auto k2 = f.small[2] ? face2_kernel<STAGE, MIX, true> : face2_kernel<STAGE, MIX, false>;
   k0<<<f.nt[0], NT3, 0, st>>>(probs, times, g, f.runs[0], f.nrun[0], f.first[0], f.nlane[0], s, f.F[0], f.own, f.all0,
                               STAGE);
   k1<<<f.nt[1], NT3, 0, st>>>(probs, times, g, f.runs[1], f.nrun[1], f.first[1], f.nlane[1], s, f.F[1], f.own, f.all0,

@@ -441,6 +441,17 @@ class Solver:
                          cur["resident"] if resident is None else resident)
         _check(library().mdg_set_launch_config(self._h, ctypes.byref(c)), "mdg_set_launch_config")
 
+    def set_run_shape(self, run_length: int = 0, small_launch: int = -1):
+        """Fix a dendritic solver's run length (0: by the grid's size) and face kernels (0 large
+        launches', 1 small launches', -1 by their size)."""
+        _check(library().mdg_set_run_shape(self._h, int(run_length), int(small_launch)), "mdg_set_run_shape")
+
+    def run_shape(self):
+        """(run length in use, bit mask of the face kernels that are the small launches')."""
+        a, b = ctypes.c_int(), ctypes.c_int()
+        _check(library().mdg_get_run_shape(self._h, ctypes.byref(a), ctypes.byref(b)), "mdg_get_run_shape")
+        return a.value, b.value
+
     def resident_cluster(self) -> int:
         """CTAs per problem of the resident stepper, 0 when mdg_step cannot use it."""
         n = ctypes.c_int()

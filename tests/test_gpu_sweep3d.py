@@ -68,6 +68,24 @@ def test_3d_one_step_from_developed_state(name):
     assert abs(t - float(g["t1"])) <= PER_STEP_TOL * float(g["t1"])
 
 
+@pytest.mark.parametrize("run,small", [(1, 0), (3, 1), (16, 0), (64, 1), (64, 0)])
+@pytest.mark.parametrize("name", sorted(k for k, (pb, _) in CASES3.items() if pb.ndim > 1))
+def test_3d_work_lists_give_the_fixture_run_bit_for_bit(name, run, small):
+    """The runs and face kernels that full-size grids take, on the fixtures' grids (whose size
+    alone gives one-face runs and the small launches' kernels): the same bits."""
+    pb, n = CASES3[name]
+    n = min(n, 40)
+    with Solver(pb) as s:
+        assert s.run_shape()[0] == 1
+        s.step(n)
+        want = s.update_cpu(0)
+        s.upload(0, pb.ic)
+        s.set_run_shape(run, small)
+        assert s.run_shape() == (run, 7 * small)
+        s.step(n)
+        assert np.array_equal(s.update_cpu(0), want)
+
+
 def test_3d_mass_change_is_the_outer_boundary_flux():
     """Reflecting inner and pole boundaries, periodic phi: mass changes only through the
     outer radial face, and the blast has not reached it."""
@@ -223,6 +241,8 @@ def test_3d_run_length_does_not_change_results(precision):
         with Solver(pb, precision=precision) as s:
             s.set_launch_config(run_length=run)
             assert s.launch_config()["run_length"] == run
+            s.set_run_shape(run_length=run)        # (this grid's size alone gives runs of one face)
+            assert s.run_shape()[0] == run
             s.step(12)
             out[run] = (s.update_cpu(0), s.time(0))
     for run in (1, 3, 64):
