@@ -113,7 +113,7 @@ struct Sweep3;
 int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why);
 void sweep3_destroy(Sweep3 *w);
 int64_t sweep3_ncell(const Sweep3 *w);
-int64_t sweep3_bytes(const Sweep3 *w);   // device memory of the grid tables, face fluxes and bits
+int64_t sweep3_bytes(const Sweep3 *w);   // device memory held: grid tables, work lists, face fluxes and bits
 // Faces per work item of the radial and theta run kernels (1..64); rebuilds the work lists.
 int sweep3_set_run_length(Sweep3 *w, int run_length, int exact, std::string &why);
 void sweep3_set_small(Sweep3 *w, int small);

@@ -309,7 +309,13 @@ struct Sweep3 {
   int nt[4] = {0, 0, 0, 0};        // CTAs of face0, face1, face2 and the zone kernels
   int ntot = 0;                    // zone tiles of the conserved totals
   int64_t ncell = 0;
-  int64_t bytes = 0;               // device memory held
+  int64_t bytes = 0;               // device memory held: every allocation goes through take()
+  template <typename T> cudaError_t take(T **p, size_t n)
+  {
+    const cudaError_t e = cudaMalloc(p, n);
+    if (e == cudaSuccess) bytes += (int64_t)n;
+    return e;
+  }
 };
 
 static void tiles_of_rows(std::vector<Tile3> &out, int i, int j, int count, int chunk = NT3)
@@ -459,9 +465,10 @@ static cudaError_t upload_runs(Sweep3 *w, int run_len, int exact)
   cudaError_t e = cudaSuccess;
   if (all.size() > w->runs_cap) {
     int *d = nullptr;
-    e = cudaMalloc(&d, sizeof(int) * all.size());
+    e = w->take(&d, sizeof(int) * all.size());
     if (e != cudaSuccess) return e;
     cudaFree(w->d_runs);
+    w->bytes -= (int64_t)(sizeof(int) * w->runs_cap);
     w->d_runs = d;
     w->runs_cap = all.size();
   }
@@ -570,8 +577,6 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     off[q] = tot;
     tot += (parts[q].second + 255) / 256 * 256;
   }
-  w->bytes = (int64_t)tot + (int64_t)sizeof(double) * NPRIM * (h.nf0 + h.nf1 + h.nf2) + 3 * h.ncell +
-             (int64_t)sizeof(double) * h.n1;
   std::vector<char> host(tot, 0);
   for (size_t q = 0; q < parts.size(); q++) std::memcpy(host.data() + off[q], parts[q].first, parts[q].second);
   auto fail3 = [&](cudaError_t e) {
@@ -581,7 +586,7 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     delete w;
     return e == cudaErrorMemoryAllocation ? MDG_ERR_OUTOFMEM : MDG_ERR_CUDA;
   };
-  cudaError_t e = cudaMalloc(&w->d_tab, tot);
+  cudaError_t e = w->take(&w->d_tab, tot);
   if (e != cudaSuccess) return fail3(e);
   e = cudaMemcpy(w->d_tab, host.data(), tot, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail3(e);
@@ -611,13 +616,13 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   g.nrow = (int)prow.size();
   g.x0 = d.startx[0];
   g.mono = d.monopole;
-  e = cudaMalloc(&w->d_gmono, sizeof(double) * (size_t)h.n1);
+  e = w->take(&w->d_gmono, sizeof(double) * (size_t)h.n1);
   if (e != cudaSuccess) return fail3(e);
   g.gmono = w->d_gmono;
   // flux arrays, shock bits
-  e = cudaMalloc(&w->d_flux, sizeof(double) * NPRIM * (size_t)(h.nf0 + h.nf1 + h.nf2));
+  e = w->take(&w->d_flux, sizeof(double) * NPRIM * (size_t)(h.nf0 + h.nf1 + h.nf2));
   if (e != cudaSuccess) return fail3(e);
-  e = cudaMalloc(&w->d_bits, (size_t)3 * h.ncell);
+  e = w->take(&w->d_bits, (size_t)3 * h.ncell);
   if (e != cudaSuccess) return fail3(e);
   e = cudaMemset(w->d_bits, 0, (size_t)3 * h.ncell);
   if (e != cudaSuccess) return fail3(e);
@@ -633,12 +638,12 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     for (int j = 0; j < h.njr(i); j++) tiles_of_rows(tc, i, j, h.nk[h.row(i, j)]);
   w->ntot = (int)tc.size();
   w->nt[3] = (int)row0.size();
-  e = cudaMalloc(&w->d_row0, sizeof(int) * row0.size());
+  e = w->take(&w->d_row0, sizeof(int) * row0.size());
   if (e != cudaSuccess) return fail3(e);
   e = cudaMemcpy(w->d_row0, row0.data(), sizeof(int) * row0.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail3(e);
   g.row0 = w->d_row0;
-  e = cudaMalloc(&w->d_tiles, sizeof(Tile3) * tc.size());
+  e = w->take(&w->d_tiles, sizeof(Tile3) * tc.size());
   if (e != cudaSuccess) return fail3(e);
   e = cudaMemcpy(w->d_tiles, tc.data(), sizeof(Tile3) * tc.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail3(e);
@@ -651,7 +656,7 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     const int *q = reinterpret_cast<const int *>(segs.data());
     all.assign(q, q + sizeof(Seg2) / sizeof(int) * segs.size());
     all.insert(all.end(), first.begin(), first.end());
-    e = cudaMalloc(&w->d_seg, sizeof(int) * all.size());
+    e = w->take(&w->d_seg, sizeof(int) * all.size());
     if (e != cudaSuccess) return fail3(e);
     e = cudaMemcpy(w->d_seg, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail3(e);

@@ -292,3 +292,22 @@ def test_server_rejects_requests(bad, code):
         with pytest.raises(MdgError) as e:
             srv.submit(pb)
         assert e.value.code == code
+
+
+def test_server_counts_all_device_memory_of_a_dendritic_request():
+    """A (r, theta) grid, whose work lists are largest against its zones: what the request takes from
+    the device, less 2 MB of rounding for each of its nine allocations, does not fit a smaller budget."""
+    import torch
+    pb = P.sedov_2d_spherical(3000, 512).copy(tmax=1.0e-6)
+    kw = dict(precision=PREC_FP64, hbm_bytes=16 << 20, max_problems=2, max_zones=128, steps_per_round=1)
+    torch.cuda.synchronize()
+    with Server(hbm_bytes_3d=8 << 30, **kw) as srv:
+        free = torch.cuda.mem_get_info()[0]
+        srv.submit(pb)
+        held = free - torch.cuda.mem_get_info()[0]
+    assert held > 200 * pb.ncell
+    with Server(hbm_bytes_3d=held - (18 << 20), **kw) as srv:
+        with pytest.raises(MdgError):
+            srv.submit(pb)
+    with Server(hbm_bytes_3d=held, **kw) as srv:
+        srv.submit(pb)
