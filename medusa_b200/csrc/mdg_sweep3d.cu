@@ -2,7 +2,6 @@
 // face kernels of both precisions are in mdg_sweep3d.cuh; the plain FP64 ones are built here.
 #include "mdg_sweep3d.cuh"
 #include <algorithm>
-#include <cstring>
 #include <string>
 #include <vector>
 
@@ -393,7 +392,10 @@ static void build_runs(const Sweep3 &w, int dir, int run_len, RunList &out)
 {
   std::vector<Run3> runs;
   std::vector<int> cnt;
+  runs.reserve(w.nk.size() / run_len);
+  cnt.reserve(w.nk.size() / run_len);
   cut_runs(w, dir, run_len, runs, cnt);
+  out.runs.reserve(runs.size());
   // long runs first (the tail of the launch is made of short ones), neighbouring rows in
   // neighbouring lanes: direction 0 by first face then theta row, direction 1 likewise
   // (a counting sort on length and first face: the runs of a pair already come in row order)
@@ -530,6 +532,8 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   std::vector<PushRow3> prow;
   std::vector<int64_t> rowcell;
   std::vector<int> row0;
+  prow.reserve((size_t)h.nij);
+  rowcell.reserve((size_t)h.nij);
   for (int i = 0; i < h.n1; i++) {
     for (int j = 0; j < h.njr(i); j++) {
       PushRow3 r{};
@@ -577,8 +581,6 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
     off[q] = tot;
     tot += (parts[q].second + 255) / 256 * 256;
   }
-  std::vector<char> host(tot, 0);
-  for (size_t q = 0; q < parts.size(); q++) std::memcpy(host.data() + off[q], parts[q].first, parts[q].second);
   auto fail3 = [&](cudaError_t e) {
     why = cudaGetErrorString(e);
     cudaFree(w->d_tab); cudaFree(w->d_flux); cudaFree(w->d_bits); cudaFree(w->d_tiles); cudaFree(w->d_gmono);
@@ -588,7 +590,9 @@ int sweep3_create(const mdg_problem_desc &d, Sweep3 **out, std::string &why)
   };
   cudaError_t e = w->take(&w->d_tab, tot);
   if (e != cudaSuccess) return fail3(e);
-  e = cudaMemcpy(w->d_tab, host.data(), tot, cudaMemcpyHostToDevice);
+  // part by part: packing them on the host first took a fifth of a (r, theta) grid's set-up
+  for (size_t q = 0; q < parts.size() && e == cudaSuccess; q++)
+    if (parts[q].second) e = cudaMemcpy(w->d_tab + off[q], parts[q].first, parts[q].second, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail3(e);
   Grid3 &g = w->g;
   g.ndim = h.ndim;
