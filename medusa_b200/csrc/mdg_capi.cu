@@ -299,6 +299,7 @@ static int build_mixed_tiles(mdg_solver *s, int nt, int lanes)
     q[2 * l + 1].ntiles = s->lane[l].ntt;
   }
   CK(cudaMemcpy(s->d_queue, q, sizeof q, cudaMemcpyHostToDevice));
+  CK(setup_landed());
   // streams and events of the extra lanes, created once
   if (s->nlanes > 1 && !s->ev_fork) {
     CK(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
@@ -433,6 +434,7 @@ static int create_3d(const mdg_problem_desc &d, int precision, int device, mdg_s
   CK3(cudaMemset(s->d_state, 0, sizeof(double) * 2 * NPRIM * n));
   CK3(cudaMemset(s->d_err, 0, sizeof(int)));
   CK3(cudaMemset(s->d_times, 0, sizeof(ProbTime)));
+  CK3(setup_landed());
   for (int v = 0; v < NPRIM; v++) {
     s->P.v[v] = s->d_state + (int64_t)v * n;
     s->PH.v[v] = s->d_state + (int64_t)(NPRIM + v) * n;
@@ -671,6 +673,7 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
   CKC(cudaMemcpy(s->d_probs, s->hprobs.data(), sizeof(ProbDev) * nprob, cudaMemcpyHostToDevice));
   CKC(cudaMemcpy(s->d_tiles, tiles.data(), sizeof(Tile) * s->ntiles, cudaMemcpyHostToDevice));
   if (dev_tables) {
+    CKC(setup_landed());   // (the records that the table kernels read)
     for (int m = 0; m < nprob; m++)
       if (!s->hprobs[m].geo_tab)
         launch_build_tables_1d(s->d_probs, m, descs[m].n1, s->d_rc0, s->d_geo, s->d_mx, rc0, s->stream);
@@ -695,6 +698,7 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
   if (ndim == 2) CKC(cudaMemset(s->d_shock0, 0, sh > 0 ? sh : 1));
   if (ndim == 2) CKC(cudaMemset(s->d_shock1, 0, sh > 0 ? sh : 1));
   CKC(cudaMemset(s->d_times, 0, sizeof(ProbTime) * nprob));
+  CKC(setup_landed());
   for (int v = 0; v < NPRIM; v++) {
     s->P.v[v] = s->d_state + (int64_t)v * cell;
     s->PH.v[v] = s->d_state + (int64_t)(NPRIM + v) * cell;
@@ -1629,6 +1633,7 @@ int mdg_eos_table_create(const mdg_eos_grid *grid, const double *table, int devi
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) ce = cudaMalloc(&t->d_f, sizeof(double) * 4 * npt);
   if (ce == cudaSuccess) ce = cudaMemcpy(t->d_f, hf.data(), sizeof(double) * 4 * npt, cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = setup_landed();
   if (ce != cudaSuccess) return bail(ce);
   *out = t;
   return MDG_OK;

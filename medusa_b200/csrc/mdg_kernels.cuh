@@ -61,6 +61,11 @@ constexpr int TIY2 = MDG_TIY2;    // most rows of a direction-1 tile
 // columns that are swept by the same launches (mdg_sweep2d.cu).
 int tile_rows_2d(int dir, const int *n1, const int *n2, int n, int num_sms);
 
+// Set-up copies and memsets run on the legacy default stream, and a copy from pageable memory may
+// return before its data have landed.  The solvers' streams are non-blocking, so nothing orders
+// them after that: every set-up ends with this wait.
+inline cudaError_t setup_landed() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 struct TmaTables1d;
 // Tabulated EOS on the device (mdg_eos_table.cu): the records f[jy][jr][jt] = {e, log p,
 // s, Gamma_1} as two double2 per grid point; grid sizes and bounds as the reference's

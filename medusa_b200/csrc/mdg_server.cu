@@ -790,6 +790,7 @@ int mdg_server_create(const mdg_server_config *cfg, mdg_server **out)
   SCKB(cudaMemset(s->d_queue, 0, 2 * sizeof(WorkQueue)));
   SCKB(cudaMemset(s->d_err, 0, sizeof(int)));
   SCKB(cudaMemset(s->d_state, 0, sizeof(double) * 2 * NPRIM * units));
+  SCKB(setup_landed());
 #undef SCKB
   for (int v = 0; v < NPRIM; v++) {
     s->P.v[v] = s->d_state + (int64_t)v * units;

@@ -475,6 +475,7 @@ static cudaError_t upload_runs(Sweep3 *w, int run_len, int exact)
     w->runs_cap = all.size();
   }
   e = cudaMemcpy(w->d_runs, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = setup_landed();
   if (e != cudaSuccess) return e;
   for (int q = 0; q < 4; q++) w->run_off[q] = off[q];
   for (int d = 0; d < 2; d++) {
