@@ -548,7 +548,13 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
   std::vector<Tile> tiles, ytiles;
   int64_t cell = 0, rc0 = 0, rc1 = 0, sh = 0;
   int xrows = TIX2, yrows = TIY2;
-  if (cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) s->num_sms = 0;
+  {
+    const cudaError_t e = cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) {
+      delete s;
+      return fail(MDG_ERR_CUDA, std::string("multiprocessor count: ") + cudaGetErrorString(e));
+    }
+  }
   if (ndim == 2) {
     std::vector<int> r1, r2;
     for (int m = 0; m < nprob; m++) { r1.push_back(descs[m].n1); r2.push_back(descs[m].n2); }
@@ -666,7 +672,6 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
     CKC(cudaMemcpy(s->d_mx, m0.data(), sizeof(float) * m0.size(), cudaMemcpyHostToDevice));
     CKC(cudaMemcpy(s->d_mx1, m1.data(), sizeof(float) * m1.size(), cudaMemcpyHostToDevice));
   }
-  CKC(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device));
   if (ndim == 2) CKC(cudaMalloc(&s->d_shock0, sh > 0 ? sh : 1));
   if (ndim == 2) CKC(cudaMalloc(&s->d_shock1, sh > 0 ? sh : 1));
 
@@ -1577,7 +1582,6 @@ int mdg_write_timers(mdg_solver *s, int prob, const char *path)
 
 struct mdg_eos_table {
   int device = 0;
-  int num_sms = 0;
   mdg_eos_grid g{};
   double2 *d_f = nullptr;
   cudaStream_t stream = nullptr;
@@ -1629,8 +1633,7 @@ int mdg_eos_table_create(const mdg_eos_grid *grid, const double *table, int devi
     if (e == cudaErrorMemoryAllocation) return fail(MDG_ERR_OUTOFMEM, "no device memory for the EOS table");
     return fail(MDG_ERR_CUDA, std::string("EOS table: ") + cudaGetErrorString(e));
   };
-  cudaError_t ce = cudaDeviceGetAttribute(&t->num_sms, cudaDevAttrMultiProcessorCount, device);
-  if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
+  cudaError_t ce = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) ce = cudaMalloc(&t->d_f, sizeof(double) * 4 * npt);
   if (ce == cudaSuccess) ce = cudaMemcpy(t->d_f, hf.data(), sizeof(double) * 4 * npt, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = setup_landed();

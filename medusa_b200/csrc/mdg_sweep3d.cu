@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(NT3, MDG_P3MINB) push3_kernel(const ProbDev *_
   const double dt = times[0].dt;
   const int64_t c = (int64_t)blockIdx.x * NT3 + threadIdx.x;
   const int row = zone_row(g, sbeg);
-  double lmin = 1.0e300, lmax = 0.0;
+  double lmin = 1.0e300;
   if (c < g.ncell) {
     const PushRow3 &pr = g.prow[row];
     const int i = pr.i, j = pr.j, ij = pr.ij, k = (int)(c - __ldg(g.rowcell + row));
@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(NT3, MDG_P3MINB) push3_kernel(const ProbDev *_
       }
     }
   }
-  (void)lmax;
   block_min_to(lmin, &times[0].minacc, sred);
 }
 
