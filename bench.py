@@ -89,6 +89,15 @@ def read_profile_value(name, key):
     return None
 
 
+def step_launches(per_step, steps, steps_per_graph, lanes=1):
+    """Kernel launches of one mdg_step call on the launched path: `per_step` a step (the stages
+    and the time update with the next dt), and one opening dt launch for every graph replay and for
+    the steps that fill no graph, each once per lane."""
+    g = steps_per_graph if 0 < steps_per_graph <= steps else 0
+    openings = steps // g + (1 if steps % g else 0) if g else 1
+    return lanes * (per_step * steps + openings)
+
+
 class ClockSampler:
     """nvidia-smi clock / throttle-reason sampling during the timed region."""
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
@@ -596,8 +605,8 @@ def run_ensemble(args, ctx):
         "config": ensemble_config(probs, ctx.world),
         "precision": "mixed: FP32 reconstruction/limiting/Riemann, FP64 state/fluxes/sources/update/dt",
         "launch": dict(tuned, autotune_ms_per_step=tune_ms),
-        # per step and lane: dt, the two stage kernels, the time update
-        "gpu_launches": 3 * K * tuned.get("lanes", 1),   # two stages, time update with the next dt
+        # per step and lane: the two stage kernels, the time update with the next dt
+        "gpu_launches": step_launches(3, K, tuned["steps_per_graph"], tuned["lanes"]),
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "mdg_run_host: upload of all %d initial states (pinned H2D) + %d steps + download of "
@@ -659,6 +668,7 @@ def run_kh(args, ctx):
     ms, clocks = timed_steps(ctx, s, K, sample_clocks=True)
     value = ctx.world * ncell * K / (ms / 1e3)
     st = stage_times(s, min(K, 20))
+    per_graph = s.launch_config()["steps_per_graph"]
     s.close()
     ms_e2e, h2d, d2h = e2e_run(ctx, lambda upload: medusa_b200.Solver(pb, device=ctx.local, upload=upload),
                                [pb], K, W)
@@ -702,7 +712,7 @@ def run_kh(args, ctx):
                    "seq_len": ncell, "parallelism": "replicas" if ctx.world > 1 else "single",
                    "precision": "plain FP64 (reference operation order)",
                    "l2": "inputs larger than L2 (state 2 x 168 MB)"},
-        "gpu_launches": 5 * K,
+        "gpu_launches": step_launches(5, K, per_graph),
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "upload initial state (pinned H2D) + %d steps + download state (pinned D2H)" % K,
@@ -795,6 +805,7 @@ def run_sedov3d(args, ctx):
     ms, clocks = timed_steps(ctx, s, K, sample_clocks=True)
     value = ctx.world * ncell * K / (ms / 1e3)
     st = stage_times(s, min(K, 10))
+    per_graph = s.launch_config()["steps_per_graph"]
     s.close()
     ms_e2e, h2d, d2h = e2e_run(ctx, lambda upload: medusa_b200.Solver(pb, device=ctx.local, upload=upload),
                                [pb], K, W)
@@ -848,7 +859,7 @@ def run_sedov3d(args, ctx):
                    "precision": "plain FP64 (reference operation order)",
                    "grid": sedov3d_grid_text(pb, args.sedov3d_radius),
                    "l2": "inputs larger than L2 (state 2 x %.0f MB)" % (ncell * 40 / 1e6)},
-        "gpu_launches": 9 * K,
+        "gpu_launches": step_launches(9, K, per_graph),
         "e2e": {"value": e2e, "unit": "zone-updates/s", "h2d_bytes_per_step": h2d / K,
                 "d2h_bytes_per_step": d2h / K,
                 "timed": "upload initial state (pinned H2D) + %d steps + download state (pinned D2H)" % K,
@@ -1092,6 +1103,7 @@ def run_sod1d(args, ctx):
         prim = s.update_cpu(0)
         t, _, istep = s.time(0)
         resident = s.resident_cluster()
+        per_graph = s.launch_config()["steps_per_graph"]
     value = ctx.world * pb.ncell * istep / (ms / 1e3)
     l1 = A.l1_rel(prim[:, 0], A.sod_exact_state(1024, t)[:, 0])
     if ctx.rank != 0:
@@ -1114,7 +1126,7 @@ def run_sod1d(args, ctx):
                    "parallelism": "replicas" if ctx.world > 1 else "single",
                    "l2": "resident in L2 (80 KB state): a latency-bound job, timed whole"},
         # resident: one launch per 256 steps; else two stages and the time update per step
-        "gpu_launches": (nmax + 255) // 256 if resident else 3 * nmax,
+        "gpu_launches": (nmax + 255) // 256 if resident else step_launches(3, nmax, per_graph),
         "resident_cluster_ctas": resident,
         "time_to_solution_ms": ms, "t": t, "clocks": clocks,
         "accuracy": dict({"l1_rho_vs_exact_riemann": l1}, **ref),

@@ -16,7 +16,7 @@
 // Small problems (at most 16 tiles, 2016 zones) can instead be advanced by the resident
 // stepper: one thread-block cluster per problem, one CTA per tile, runs the whole step
 // sequence of many steps in one launch -- the dt rules, both RK stages and the time
-// update, separated by cluster barriers -- where the per-phase path pays four dependent
+// update, separated by cluster barriers -- where the per-phase path pays three dependent
 // launches per step.  It runs the same tile code, so the two paths agree bit for bit.
 #include "mdg_hydro.cuh"
 #include "mdg_kernels.cuh"

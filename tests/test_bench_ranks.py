@@ -63,3 +63,11 @@ def test_two_gloo_ranks_partition_and_reduce():
     # each rank has its own ensemble and its own request stream
     assert res[0][5] != res[1][5]
     assert res[0][6] != res[1][6]
+
+
+@pytest.mark.parametrize("args,want", [((3, 20, 10), 62), ((3, 25, 10, 2), 156), ((5, 7, 10), 36), ((9, 10, 10), 91),
+                                       ((3, 12, 0), 37)])
+def test_launch_count_includes_the_opening_dt_launches(args, want):
+    """Per step the stages and the time update; one dt launch more per graph replay, for the
+    remaining steps, and per lane."""
+    assert bench.step_launches(*args) == want
