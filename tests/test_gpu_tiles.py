@@ -32,6 +32,27 @@ def test_2d_tile_edges_match_the_oracle(kind, n1, n2):
     assert pointwise_rel_err(got, ref, pb) <= 1.0e-12 * steps
 
 
+# The mixed sweep on the same edges, against the plain FP64 oracle: FP32 face states and star-state
+# increments carry 6e-8 of rho v^2 + p (mdg_mixed.cuh), a few of them a zone and stage, and the blast's
+# declined faces are solved again in FP64 from the tables.
+@pytest.mark.parametrize("n1,n2", [(5, 4), (33, 127), (64, 126), (67, 129), (130, 253), (515, 260), (1030, 300)])
+@pytest.mark.parametrize("kind", ["kh", "blast"])
+def test_2d_tile_edges_mixed(kind, n1, n2):
+    pb = P.kelvin_helmholtz(n1, n2) if kind == "kh" else P.blast_2d(n1, n2, bc=P.REFLECT)
+    steps = 2
+    with Solver(pb, precision=PREC_MIXED) as s:
+        s.step(steps)
+        s.synchronize()
+        got = s.update_cpu(0)
+    o = pyoracle.Oracle(pb)
+    o.advance(steps)
+    ref, _ = o.state()
+    assert np.all(np.isfinite(got))
+    assert field_rel_err(got[:, :2], ref[:, :2]) <= 1.0e-6 * steps
+    vscale = max(np.abs(ref[:, 2:4]).max(), np.sqrt(pb.gam * (pb.gam - 1.0) * ref[:, 1] / ref[:, 0]).max())
+    assert np.abs(got[:, 2:5] - ref[:, 2:5]).max() <= 1.0e-6 * steps * vscale
+
+
 # 2-D rows of one phi zone (a last CTA with idle lanes), small 3-D rows several to a CTA, rows
 # of 128 phi zones (cut segments)
 @pytest.mark.parametrize("dims", [(71, 64, 1), (33, 16, 32), (60, 64, 128)])
