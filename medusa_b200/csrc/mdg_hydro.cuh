@@ -499,8 +499,8 @@ __device__ __forceinline__ double eos_press(int eos, double gam, double Kpoly, d
   return (eos == 0) ? (gam - 1.0) * uu : Kpoly * pow(rho, gam);
 }
 
-// Smallest of a full warp's keys: the integer reduction unit on the high and then the low words
-// (4 instructions for the 25 of a shuffle tree of doubles).
+// Smallest of a full warp's keys: the integer reduction unit on the high and then the low words,
+// in place of a five-step shuffle tree of doubles.
 __device__ __forceinline__ unsigned long long warp_min_ord(unsigned long long k)
 {
   const unsigned h = (unsigned)(k >> 32), hm = __reduce_min_sync(0xffffffffu, h);

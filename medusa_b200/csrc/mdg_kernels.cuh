@@ -47,8 +47,8 @@ constexpr int TILE1 = NT1 - 2;
 #ifndef MDG_YMINB
 #define MDG_YMINB 4
 #endif
-// (mixed sweep at 2048^2: 1.48 ms per step with 3 CTAs of 168 registers, 1.54 with 4, 1.88 with 2;
-// plain FP64 2.80 ms with 4, 3.10 ms with 3)
+// (mixed sweep at 2048^2: 1.48 ms per step with 3 CTAs of 168 registers, 1.53 with 4, 1.89 with 2;
+// plain FP64 2.69 ms with 4 CTAs in direction 1, 2.88 ms with 3)
 #ifndef MDG_MIX2_MINB
 #define MDG_MIX2_MINB 3
 #endif

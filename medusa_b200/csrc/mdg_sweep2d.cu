@@ -8,11 +8,13 @@ namespace mdg {
 // its rows (and of what it does once: two more reconstructed rows in direction 0, the
 // column tables in direction 1), and a row takes a nearly fixed time while few CTAs share
 // an SM (a chain of dependent FP64 operations) and a time that grows with them once four
-// do.  Measured on a B200, plain FP64: a direction-0 row 6.5 us alone on its SM and 11 us
-// beside three others, a direction-1 row 13 us and 14 us.  The count with the smallest
-// modelled time is taken: full-size grids keep the longest tiles (2048^2: 32 and 16 rows),
-// small ones are cut until the chip is full -- 512^2 with 32 and 16 rows gave 64 and 160
-// CTAs for 592 places, and a step took 1.0 ms.
+// do.  Measured on a B200 when the rule was made, plain FP64 with the dividing reconstruction: a
+// direction-0 row 6.5 us alone on its SM and 11 us beside three others, a direction-1 row 13 us
+// and 14 us; the kernels are faster since, and the rule was not measured again.  The count
+// with the smallest modelled time is taken: full-size grids keep long tiles (2048^2: 32 and 15
+// rows), small ones are cut until the chip is full -- 512^2 with 32 and 16 rows gave 64 and 160
+// CTAs for 592 places, and a step took 1.0 ms (0.268 ms now, 296 and 515 CTAs).  The mixed sweep,
+// whose kernels hold 3 CTAs per SM, takes the same tiles.
 int tile_rows_2d(int dir, const int *n1, const int *n2, int n, int num_sms)
 {
   const int most = dir ? TIY2 : TIX2, cols = dir ? TJY2 : NTX2;

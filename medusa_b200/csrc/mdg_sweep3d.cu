@@ -377,9 +377,10 @@ static void cut_runs(const Sweep3 &w, int dir, int run_len, std::vector<Run3> &r
 // Longest run, up to run_len faces, for which the grid's lanes still fill the chip (5 CTAs of
 // 128 lanes on every SM).  What a lane does once, three pencil entries and a reconstruction,
 // is about two faces' worth, so long runs pay where there are lanes enough: ms per step on a
-// B200 for runs of 1 / 4 / 8 / 16, 2-D 400 x 256 mixed 0.206 / 0.287 / 0.419 / 0.712 (taken: 1),
-// 3-D 100 x 32 x 64 plain FP64 0.581 / 0.693 / 0.856 / 1.287 (1), 128 x 64 x 128 plain FP64 1.971 /
-// 1.802 / 1.695 / 2.179 (8), 384 x 128 x 256 plain FP64 11.55 / 9.07 / 8.60 / 8.46 (16).
+// B200 for runs of 1 / 4 / 8 / 16, 2-D 400 x 256 mixed 0.165 / 0.233 / 0.327 / 0.532 (taken: 1),
+// 3-D 100 x 32 x 64 plain FP64 0.416 / 0.456 / 0.578 / 0.867 (1), 128 x 64 x 128 plain FP64 1.547 /
+// 1.342 / 1.245 / 1.538 (8), 384 x 128 x 256 plain FP64 9.13 / 7.24 / 6.85 / 6.70 and mixed 7.47 / 5.74 /
+// 5.41 / 5.25 (16).
 static int fitting_run(const Sweep3 &w, int run_len)
 {
   const int64_t fill = (int64_t)(w.num_sms > 0 ? w.num_sms : 148) * 5 * NT3;

@@ -41,9 +41,9 @@ struct Tile3 { int i, j, k0, cnt; };
 constexpr int NT3 = 128;
 // resident CTAs per SM requested from the compiler (register caps).  The face kernels wait
 // on dependent gathers and on FP64 latency; ms per step on a B200 with 8 / 6 / 5 / 4 CTAs of
-// 128 threads (64 / 80 / 96 / 128 registers): plain FP64 384 x 128 x 256 7.53 / 7.10 / 7.28 /
-// 7.84, 128 x 64 x 128 1.49 / 1.39 / 1.63 / 1.62; mixed 384 x 128 x 256 5.97 (8), 5.87 (7 and 6),
-// 6.07 (5), 6.55 (4).
+// 128 threads (64 / 80 / 96 / 128 registers): plain FP64 384 x 128 x 256 6.95 / 6.62 / 6.75 /
+// 7.37, 128 x 64 x 128 1.37 / 1.24 / 1.47 / 1.46; mixed 384 x 128 x 256 with 8 / 7 / 6 / 5 / 4
+// 5.41 / 5.27 / 5.31 / 5.44 / 5.91.
 #ifndef MDG_F3MINB
 #define MDG_F3MINB 6
 #endif
@@ -52,7 +52,8 @@ constexpr int NT3 = 128;
 #endif
 // Launches of at most F3MINB_SMALL CTAs per SM are all resident with 96 registers a thread as
 // well, which leaves fewer spills on the chain of one thread's operations: 2-D 400 x 256 blast,
-// 725 CTAs, plain FP64 210 -> 191 us per step, mixed 207 -> 161 us.
+// 725 CTAs, plain FP64 202 -> 187 us per step, mixed 203 -> 164 us (384 x 128 x 256 with them: 6.69 ->
+// 6.86 ms, mixed 5.25 -> 5.46).
 constexpr int F3MINB_SMALL = 5;
 constexpr int f3_minb(bool mix, bool small) { return small ? F3MINB_SMALL : mix ? MDG_F3MINB_MIX : MDG_F3MINB; }
 #ifndef MDG_P3MINB
