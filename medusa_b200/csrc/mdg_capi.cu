@@ -1582,6 +1582,7 @@ int mdg_write_timers(mdg_solver *s, int prob, const char *path)
 
 struct mdg_eos_table {
   int device = 0;
+  int num_sms = 0;
   mdg_eos_grid g{};
   double2 *d_f = nullptr;
   cudaStream_t stream = nullptr;
@@ -1633,7 +1634,8 @@ int mdg_eos_table_create(const mdg_eos_grid *grid, const double *table, int devi
     if (e == cudaErrorMemoryAllocation) return fail(MDG_ERR_OUTOFMEM, "no device memory for the EOS table");
     return fail(MDG_ERR_CUDA, std::string("EOS table: ") + cudaGetErrorString(e));
   };
-  cudaError_t ce = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
+  cudaError_t ce = cudaDeviceGetAttribute(&t->num_sms, cudaDevAttrMultiProcessorCount, device);
+  if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking);
   if (ce == cudaSuccess) ce = cudaMalloc(&t->d_f, sizeof(double) * 4 * npt);
   if (ce == cudaSuccess) ce = cudaMemcpy(t->d_f, hf.data(), sizeof(double) * 4 * npt, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = setup_landed();
@@ -1650,7 +1652,7 @@ int mdg_eos_given_rex(mdg_eos_table *t, long long n, const double *rho, const do
   if (n > 0 && (!rho || !u || !ye || !temp || !press || !cs || !ent || !gam1))
     return fail(MDG_ERR_INVALID, "null zone array");
   CK(cudaSetDevice(t->device));
-  launch_eos_rex(t->dev(), n, rho, u, ye, temp, press, cs, ent, gam1, (cudaStream_t)stream);
+  launch_eos_rex(t->dev(), n, rho, u, ye, temp, press, cs, ent, gam1, t->num_sms, (cudaStream_t)stream);
   CK(cudaGetLastError());
   return MDG_OK;
 }
@@ -1674,7 +1676,7 @@ int mdg_eos_given_rex_host(mdg_eos_table *t, long long n, const double *rho, con
   for (int k = 0; k < 4 && e == cudaSuccess; k++)
     e = cudaMemcpyAsync(dz[k], hin[k], b, cudaMemcpyHostToDevice, t->stream);
   if (e == cudaSuccess) {
-    launch_eos_rex(t->dev(), n, dz[0], dz[1], dz[2], dz[3], dz[4], dz[5], dz[6], dz[7], t->stream);
+    launch_eos_rex(t->dev(), n, dz[0], dz[1], dz[2], dz[3], dz[4], dz[5], dz[6], dz[7], t->num_sms, t->stream);
     e = cudaGetLastError();
   }
   double *dout[5] = {dz[3], dz[4], dz[5], dz[6], dz[7]};

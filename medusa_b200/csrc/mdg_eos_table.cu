@@ -23,10 +23,12 @@
 
 namespace mdg {
 
-// 256 threads, 4 CTAs per SM (64 registers), a thread per zone: 4 M zones on a B200, L2 flushed
-// between calls (8 CTAs of 256 threads per SM in a grid-stride loop before): guesses from the last
-// step 0.447 -> 0.426 ms, a row too high 0.444 -> 0.424, a row too low 0.506 -> 0.490.
-constexpr int EOS_NT = 256;
+// 256 threads, 4 CTAs per SM (64 registers), at most 16 CTAs per SM in the grid.  Before: 8 CTAs per
+// SM in the grid and no register cap.  On a B200, L2 flushed between calls, 4 M zones with guesses
+// from the last step 448 -> 420 us, a few per cent off 447 -> 430, a row too high 444 -> 418, a row
+// too low 506 -> 486; 1 M zones 128 -> 128, 130 -> 132, 126 -> 128, 142 -> 142; 200 k and 20 k zones
+// within 1 us.  A thread per zone: 425 / 451 / 424 / 492 us and, 1 M, 126 / 133 / 124 / 141.
+constexpr int EOS_NT = 256, EOS_CTAS = 16;
 
 __global__ void __launch_bounds__(EOS_NT, 4)
 eos_rex_kernel(EosTableDev d, long long n, const double *__restrict__ rho, const double *__restrict__ u,
@@ -87,9 +89,9 @@ eos_rex_kernel(EosTableDev d, long long n, const double *__restrict__ rho, const
       return e;
     };
 
-    // (Both rows read at once are faster for guesses from the last step, 4 M zones 404 for 426 us,
-    // but a guess that lies a row or two too high has then read a row in vain: 469 for 424 us and
-    // 522 for 490 us.)
+    // (Both rows read at once are faster for guesses from the last step, 4 M zones 404 us, but a guess
+    // that lies a row or two too high has then read a row in vain: 469 us and 522 us, more than
+    // before.)
     double elo, ehi = -1e99;
     while (true) {
       elo = energy(jt);
@@ -146,11 +148,12 @@ eos_rex_kernel(EosTableDev d, long long n, const double *__restrict__ rho, const
 }
 
 void launch_eos_rex(const EosTableDev &d, long long n, const double *rho, const double *u, const double *ye,
-                    double *temp, double *press, double *cs, double *ent, double *gam1, cudaStream_t st)
+                    double *temp, double *press, double *cs, double *ent, double *gam1, int num_sms,
+                    cudaStream_t st)
 {
   if (n <= 0) return;
   const long long blocks = (n + EOS_NT - 1) / EOS_NT;
-  const long long cap = 0x7fffffffll;
+  const long long cap = (long long)(num_sms > 0 ? num_sms : 148) * EOS_CTAS;
   const int grid = (int)(blocks < cap ? blocks : cap);
   eos_rex_kernel<<<grid, EOS_NT, 0, st>>>(d, n, rho, u, ye, temp, press, cs, ent, gam1);
 }

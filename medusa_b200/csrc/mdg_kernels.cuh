@@ -76,7 +76,8 @@ struct EosTableDev {
   double r1, r2, t1, t2, y1, y2, const_hack;
 };
 void launch_eos_rex(const EosTableDev &d, long long n, const double *rho, const double *u, const double *ye,
-                    double *temp, double *press, double *cs, double *ent, double *gam1, cudaStream_t st);
+                    double *temp, double *press, double *cs, double *ent, double *gam1, int num_sms,
+                    cudaStream_t st);
 // The resident 1-D stepper (plain FP64): CTAs per problem for problems of at most
 // max_tiles tiles (a power of two), or 0 when it cannot run (more than
 // RESIDENT1D_MAX_TILES tiles, or such a cluster does not fit this device), and whether nprob

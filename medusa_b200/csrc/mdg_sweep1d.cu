@@ -8,7 +8,7 @@
 // they are produced on load by the boundary kinds of reset_boundaries_gpu (bc.c:705-1422)
 // as index maps.  The CFL minimum (face terms step.c:560, source terms step.c:393, and in
 // the second stage the zone terms of the next estimate_dt, step.c:177-187) is reduced
-// per CTA with warp shuffles and folded into the problem's accumulator with one atomic.
+// per CTA by warp reductions and folded into the problem's accumulator with one atomic.
 //
 // Many problems of different sizes are advanced by one launch: the grid is a list of
 // (problem, tile) work items.
