@@ -87,7 +87,7 @@ struct mdg_solver {
   // plain FP64 1-D solvers without monopole gravity whose problems have at most
   // RESIDENT1D_MAX_TILES tiles: CTAs per problem of the resident stepper (0: none)
   int res_cs = 0;
-  bool res_wide = false;  // ... with four threads per zone
+  Resident1d res_kind = Resident1d::narrow;   // ... and its kernel
   // CUDA graph of cfg.steps_per_graph steps (rebuilt when the launch shape changes)
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
@@ -731,7 +731,7 @@ int mdg_create(const mdg_problem_desc *descs, int nprob, int precision, int devi
   if (precision == MDG_PREC_FP64 && ndim == 1 && !s->any_mono) {
     int max_tiles = 0;
     for (const ProbDev &P : s->hprobs) max_tiles = std::max(max_tiles, (P.n1 + TILE1 - 1) / TILE1);
-    s->res_cs = resident1d_cluster_size(max_tiles, s->nprob, &s->res_wide);
+    s->res_cs = resident1d_cluster_size(max_tiles, s->nprob, &s->res_kind);
   }
   *out = s;
   return MDG_OK;
@@ -983,7 +983,7 @@ int mdg_step(mdg_solver *s, int nsteps)
   CK(cudaSetDevice(s->device));
   if (uses_resident(s)) {
     for (int left = nsteps; left > 0; left -= RESIDENT_STEPS)
-      CK(launch_resident1d(s->res_cs, s->res_wide, s->nprob, s->d_probs, s->d_times, s->tb, s->P, s->PH,
+      CK(launch_resident1d(s->res_cs, s->res_kind, s->nprob, s->d_probs, s->d_times, s->tb, s->P, s->PH,
                            std::min(left, RESIDENT_STEPS), s->d_err, s->stream));
     return MDG_OK;
   }

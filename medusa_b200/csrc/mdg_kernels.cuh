@@ -80,14 +80,15 @@ void launch_eos_rex(const EosTableDev &d, long long n, const double *rho, const 
                     cudaStream_t st);
 // The resident 1-D stepper (plain FP64): CTAs per problem for problems of at most
 // max_tiles tiles (a power of two), or 0 when it cannot run (more than
-// RESIDENT1D_MAX_TILES tiles, or such a cluster does not fit this device), and whether nprob
-// such problems can have four threads per zone (wide); the launch of nsteps steps of nprob
-// problems with that cluster size.
+// RESIDENT1D_MAX_TILES tiles, or such a cluster does not fit this device), and the kernel for
+// nprob such problems: one thread per zone with 3 or 4 CTAs per SM, or four threads per zone;
+// the launch of nsteps steps of nprob problems with that cluster size and kernel.
 constexpr int RESIDENT1D_MAX_TILES = 16;
 constexpr int RESIDENT_STEPS = 256;   // most steps of one launch
-int resident1d_cluster_size(int max_tiles, int nprob, bool *wide);
-cudaError_t launch_resident1d(int cs, bool wide, int nprob, const ProbDev *probs, ProbTime *times, const Tables &tb,
-                              StateSoA p, StateSoA ph, int nsteps, int *err, cudaStream_t st);
+enum class Resident1d { narrow, dense, wide };
+int resident1d_cluster_size(int max_tiles, int nprob, Resident1d *kind);
+cudaError_t launch_resident1d(int cs, Resident1d kind, int nprob, const ProbDev *probs, ProbTime *times,
+                              const Tables &tb, StateSoA p, StateSoA ph, int nsteps, int *err, cudaStream_t st);
 // One RK stage of the plain FP64 1-D sweep; tm (may be NULL): tensor maps of tb's rc0 and
 // geo tables, with which each tile's tables are staged into shared memory by TMA.
 void launch_stage1d(int stage, const ProbDev *probs, ProbTime *times, const Tile *tiles, int ntiles,

@@ -274,8 +274,11 @@ stage1d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times,
 // clusters resident at once) the groups run them side by side.  Together with the record
 // copies (two barriers a step for three, no thread that the others wait for): Sod 1024 23.5 ->
 // 21.1 us per step.
-template <int G>
-__global__ void __launch_bounds__(NT1 * G, G > 1 ? 1 : 3)
+//
+// PER_SM: CTAs per SM asked of the compiler.  One thread per zone comes with 3 (162 registers) and
+// with 4 (128), see resident1d_cluster_size.
+template <int G, int PER_SM>
+__global__ void __launch_bounds__(NT1 * G, PER_SM)
 resident1d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ times, Tables tb, StateSoA p,
                   StateSoA ph, int nsteps, int *err, const __grid_constant__ TmaTables1d none)
 {
@@ -330,11 +333,20 @@ resident1d_kernel(const ProbDev *__restrict__ probs, ProbTime *__restrict__ time
   cl.sync();                                               // the CTAs' words outlive every reader
 }
 
-static cudaLaunchConfig_t resident1d_config(int cs, int nprob, bool wide, cudaStream_t st, cudaLaunchAttribute *attr)
+static void (*resident1d_fn(Resident1d kind))(const ProbDev *, ProbTime *, Tables, StateSoA, StateSoA, int, int *,
+                                              const TmaTables1d)
+{
+  return kind == Resident1d::wide    ? resident1d_kernel<4, 1>
+         : kind == Resident1d::dense ? resident1d_kernel<1, 4>
+                                     : resident1d_kernel<1, 3>;
+}
+
+static cudaLaunchConfig_t resident1d_config(int cs, int nprob, Resident1d kind, cudaStream_t st,
+                                            cudaLaunchAttribute *attr)
 {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)(cs * nprob), 1, 1);
-  c.blockDim = dim3(wide ? 4 * NT1 : NT1, 1, 1);
+  c.blockDim = dim3(kind == Resident1d::wide ? 4 * NT1 : NT1, 1, 1);
   c.dynamicSmemBytes = 0;
   c.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -347,15 +359,15 @@ static cudaLaunchConfig_t resident1d_config(int cs, int nprob, bool wide, cudaSt
 }
 
 // Clusters of cs CTAs that the device holds at once (0: none, or the query failed).
-static int resident1d_clusters(int cs, bool wide)
+static int resident1d_clusters(int cs, Resident1d kind)
 {
-  const void *f = wide ? (const void *)resident1d_kernel<4> : (const void *)resident1d_kernel<1>;
+  const void *f = (const void *)resident1d_fn(kind);
   if (cs > 8 && cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t c = resident1d_config(cs, 1, wide, nullptr, attr);
+  const cudaLaunchConfig_t c = resident1d_config(cs, 1, kind, nullptr, attr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, f, &c) != cudaSuccess) {
     cudaGetLastError();
@@ -364,29 +376,35 @@ static int resident1d_clusters(int cs, bool wide)
   return n;
 }
 
-int resident1d_cluster_size(int max_tiles, int nprob, bool *wide)
+int resident1d_cluster_size(int max_tiles, int nprob, Resident1d *kind)
 {
-  *wide = false;
+  *kind = Resident1d::narrow;
   if (max_tiles < 1 || max_tiles > RESIDENT1D_MAX_TILES) return 0;
   int cs = 1;
   while (cs < max_tiles) cs <<= 1;
-  if (resident1d_clusters(cs, false) < 1) return 0;
+  const int narrow = resident1d_clusters(cs, Resident1d::narrow), dense = resident1d_clusters(cs, Resident1d::dense);
+  if (narrow < 1 && dense < 1) return 0;
+  // One thread per zone: the clusters run in waves, so 4 CTAs per SM where that takes fewer waves,
+  // else the 3 whose 162 registers are 3-8 % faster.  us per step on a B200, 3 and 4 CTAs per SM: 592
+  // problems of up to 126 zones 58 / 38, 48 of up to 1500 (16 CTAs each) 80 / 61, 37 of up to 2000 58 / 64, 100
+  // of up to 480 30.0 / 31.1, 12 of up to 250 24.8 / 25.4.
+  auto waves = [&](int held) { return held < 1 ? nprob + 1 : (nprob + held - 1) / held; };
+  if (waves(dense) < waves(narrow)) *kind = Resident1d::dense;
   // four threads per zone, a whole SM per CTA, for up to 16 CTAs: a ninth of the device, so that
   // several solvers can run beside each other.  (Four solvers of 9 problems of 91-450 zones, 36
   // CTAs each, took 46 us a step that way and 30 us with one thread per zone.)
-  *wide = cs * nprob <= 16 && resident1d_clusters(cs, true) >= nprob;
+  if (cs * nprob <= 16 && resident1d_clusters(cs, Resident1d::wide) >= nprob) *kind = Resident1d::wide;
   return cs;
 }
 
-cudaError_t launch_resident1d(int cs, bool wide, int nprob, const ProbDev *probs, ProbTime *times, const Tables &tb,
-                              StateSoA p, StateSoA ph, int nsteps, int *err, cudaStream_t st)
+cudaError_t launch_resident1d(int cs, Resident1d kind, int nprob, const ProbDev *probs, ProbTime *times,
+                              const Tables &tb, StateSoA p, StateSoA ph, int nsteps, int *err, cudaStream_t st)
 {
   if (nsteps <= 0 || nprob <= 0) return cudaSuccess;
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t c = resident1d_config(cs, nprob, wide, st, attr);
+  const cudaLaunchConfig_t c = resident1d_config(cs, nprob, kind, st, attr);
   static const TmaTables1d none{};
-  if (wide) return cudaLaunchKernelEx(&c, resident1d_kernel<4>, probs, times, tb, p, ph, nsteps, err, none);
-  return cudaLaunchKernelEx(&c, resident1d_kernel<1>, probs, times, tb, p, ph, nsteps, err, none);
+  return cudaLaunchKernelEx(&c, resident1d_fn(kind), probs, times, tb, p, ph, nsteps, err, none);
 }
 
 void launch_stage1d(int stage, const ProbDev *probs, ProbTime *times, const Tile *tiles, int ntiles,

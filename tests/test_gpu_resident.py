@@ -119,3 +119,17 @@ def test_resident_off_with_timers_and_invalid_setting():
         assert s.timers()["stage0"][1] == 10
         with pytest.raises(MdgError):
             s.set_launch_config(resident=2)
+
+
+@pytest.mark.parametrize("per_sm,n1", [(4, 126), (4, 60), (2, 300)])
+def test_resident_of_more_clusters_than_three_per_sm_equals_per_phase(per_sm, n1):
+    """As many CTAs as fit at four per SM, and clusters of four: the kernel with fewer registers."""
+    import torch
+    count = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    pbs = [P.spherical_1d(("sod", "noh", "sedov")[m % 3], n1 - m % 7, 1.4) for m in range(count)]
+    cs, res = _run(pbs, 60, 1)
+    assert cs == {60: 1, 126: 1, 300: 4}[n1]
+    _, ref = _run(pbs, 60, 0)
+    for a, b in zip(res, ref):
+        assert np.array_equal(a[0], b[0], equal_nan=True)
+        assert np.array_equal(a[1], b[1], equal_nan=True)
