@@ -6,6 +6,8 @@ import itertools
 import numpy as np
 import pytest
 
+from medusa_b200 import problems as P
+from medusa_b200.solver import PREC_FP64, PREC_MIXED, Solver
 from tests import _device
 
 pytestmark = pytest.mark.gpu
@@ -113,3 +115,40 @@ def test_fp64_quotients_by_one_reciprocal(mixed):
     else:
         assert np.array_equal(got, want, equal_nan=True)
         assert np.array_equal(np.signbit(got) | np.isnan(got), np.signbit(want) | np.isnan(want))
+
+
+def _mixed_errors(batches, steps):
+    """Geometric mean over all problems of the mixed sweep's relative error (2-norm) of density and
+    internal energy against the plain FP64 sweep after the same steps."""
+    e = []
+    for pbs in batches:
+        state = []
+        for prec in (PREC_FP64, PREC_MIXED):
+            with Solver(pbs, precision=prec) as s:
+                s.step(steps)
+                s.synchronize()
+                state.append([s.update_cpu(m) for m in range(len(pbs))])
+        for a, b in zip(*state):
+            e.append([np.linalg.norm(b[:, v] - a[:, v]) / np.linalg.norm(a[:, v]) for v in (0, 1)])
+    return np.exp(np.mean(np.log(np.array(e) + 1.0e-18), axis=0))
+
+
+# What the sweeps had with correctly rounded quotients and roots, without contraction: (density,
+# internal energy).  Over such samples the means of two builds differ by up to a tenth, so a bar of 1.25.
+ROUNDED = {"ensemble": (1.670e-8, 3.911e-8), "shear": (1.233e-8, 1.992e-8), "blast2d": (2.650e-9, 1.785e-8),
+           "blast3d": (2.105e-9, 8.992e-9)}
+SAMPLES = {
+    "ensemble": (lambda: [P.ensemble_1d(96, seed=21, nmin=100, nmax=2000)], 40),
+    "shear": (lambda: [[P.kelvin_helmholtz(70 + 53 * i, 60 + 61 * (i * 5 % 8))] for i in range(6)], 60),
+    "blast2d": (lambda: [[P.sedov_2d_spherical(80 + 37 * i, (32, 64, 128)[i % 3], noise=0.01, r_dep=0.05)]
+                         for i in range(6)], 60),
+    "blast3d": (lambda: [[P.sedov_3d(50 + 11 * i, (16, 32)[i % 2], (32, 64)[i % 2], noise=0.01, r_dep=0.1)]
+                         for i in range(6)], 60),
+}
+
+
+@pytest.mark.parametrize("kind", sorted(SAMPLES))
+def test_mixed_sweeps_are_as_near_to_fp64_as_with_rounded_operations(kind):
+    make, steps = SAMPLES[kind]
+    got = _mixed_errors(make(), steps)
+    assert np.all(got <= 1.25 * np.array(ROUNDED[kind])), got
